@@ -252,6 +252,98 @@ CH_HD float floor_frac_small(float x, int &ix) {
     return x - r;
 }
 
+// ---- one f32 addition per sample coordinate ---------------------------------------
+// A target sample's coordinate is x = RN32(RN64(g + d) - 0.25) with g = a tap's global-warp
+// position / 2 (f32), d = the hypothesis's displacement / 2 (f64, at most 64 in magnitude).
+// The subtraction is exact (s = RN64(g + d) >= 0.25 is a multiple of its ulp, and so is the
+// result). grid_offset finds an f32 offset e with RN32(g + e) = x for every tap of a patch,
+// so a tap costs one f32 addition per coordinate instead of two f64 additions and a
+// conversion. It is the classical innocuous double rounding by rounding to odd (Boldo and
+// Melquiond, 2008), on the grid of the patch:
+//   Let g_lowest be the smallest g of the patch and `lowest` the smallest x, its own or a few
+//   ulps less (both positive), and w = min(ulp(lowest) / 4, ulp(g_lowest) / 2). Every g is a multiple of 2 w, and every
+//   midpoint between two floats >= lowest is a multiple of 2 w. Write d - 0.25 = (r + f) w
+//   with r an integer and 0 <= f < 1, and e = (r | 1) w, or r w when f = 0.
+//   f = 0: g + e is g + d - 0.25 itself, which is a multiple of w, so s is exact and one
+//   rounding is left on both sides.
+//   0 < f < 1: g + d - 0.25 lies strictly between two neighbouring multiples of w, one of
+//   which, the odd one, is g + e. No midpoint lies between or on the odd one, so both round
+//   to the same float. s differs from g + d by at most 2^-41 (s < 2^13: planes of at most
+//   8192 pixels a side, the caller's check), which is below 2^-20 w at w >= 2^-20; f within
+//   2^-19 of 0 or 1 is refused, so s - 0.25 stays between the two multiples as well.
+// e must be an f32: |r| + 1 < 2^24. Returns false where a condition fails (a patch within 32
+// pixels of the left or top edge, mostly); the caller then adds in f64.
+constexpr int GRID_OFFSET_MAX_SIDE = 8192;
+
+CH_HD bool grid_offset(double d, float g_lowest, float &e) {
+    const double shift = d - 0.25;
+    const float lowest = g_lowest + (float)shift;  // within 4 ulps where it is at least 32
+    const int ex = ((int32_t)f2u(lowest) - 8) >> 23, eg = (int32_t)f2u(g_lowest) >> 23;  // negative: below 0
+    const int k = ex - 25 < eg - 24 ? ex - 25 : eg - 24;                                 // w = 2^(k - 127)
+    if (k < 107) return false;                                                           // w >= 2^-20
+    // r + f. d - 0.25 rounds only where |d| < 1/8, by at most 2^-55: far less than 2^-19 w, and
+    // where it lands on a multiple of w, s rounds to that multiple + 0.25 too (s >= 32)
+    const double q = shift * u2d((uint64_t)(1023 + 127 - k) << 52);
+    if (!(fabs(q) < 16777214.0)) return false;
+#ifdef __CUDA_ARCH__
+    const double m = __dadd_rd(q, 6755399441055744.0);  // 1.5 * 2^52: the low word holds floor(q)
+    const int r = __double2loint(m);
+    const double f = q - (m - 6755399441055744.0);
+#else
+    const double floor_q = std::floor(q);
+    const int r = (int)floor_q;
+    const double f = q - floor_q;
+#endif
+    constexpr double edge = 0x1p-19;
+    if (f != 0.0 && !(f > edge && f < 1.0 - edge)) return false;
+    uint32_t w = (uint32_t)k << 23;
+    float wf;
+    memcpy(&wf, &w, 4);
+    e = (float)(f != 0.0 ? r | 1 : r) * wf;
+    return true;
+}
+
+#ifdef __CUDACC__
+// ---- packed f32 pairs -------------------------------------------------------------
+// Two IEEE f32 operations in one instruction (add, add rounded down, multiply, fused
+// multiply-add), each element rounded by itself. ptxas contracts a packed product and a packed
+// sum into a fused one whatever their rounding modifiers and -fmad say (checked on the device),
+// so a sum of products is written add2_products, with a factor of one it cannot see through.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2_down(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rm.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+// a + b for products a and b; `one` is (1, 1) in a value that reaches the kernel from outside.
+__device__ __forceinline__ f32x2 add2_products(f32x2 a, f32x2 b, f32x2 one) { return fma2(a, one, b); }
+#endif
+
 // ---- Plane::sample (image.rs:451-466) --------------------------------------------
 struct PlaneRef {
     const float *data;
@@ -319,6 +411,7 @@ CH_HD bool warp_map(const WarpRef &w, float x, float y, float &qx, float &qy) {
 struct DevCamera {
     double k[9], k_inverse[9];
     double dist_center[2], dist_norm[2], dist_coeffs[5];
+    double dist_norm_inverse[2];  // RN(1 / dist_norm), 0 where div_by does not apply
     double rotation_wc[9], rotation_cw[9], translation_wc[3], center[3];
     double real_cw[9], reflect[9], virtual_center[3];
     double oc[9];
@@ -351,9 +444,22 @@ CH_HD void distort_normalized(const double *c, double x, double y, double &ox, d
     oy = y * radial + p1 * (r2 + 2.0 * y * y) + 2.0 * p2 * x * y;
 }
 
+// RN(a / b) for a divisor whose reciprocal y = RN(1 / b) is at hand: two residual corrections of
+// a y (Markstein, IA-64 and Elementary Functions, 2000, theorem 8.2: with y correctly rounded and
+// q a faithful quotient, q + (a - b q) y rounds to a / b). The first correction makes the
+// quotient faithful. b is within [2^-500, 2^500] (else y = 0 and the division is done), and a
+// quotient that is not normal (a below 2^-500) differs from 0 by nothing a pixel could show. A
+// caller sees NaN instead of an infinity for an infinite a; both end as no projection.
+CH_HD double div_by(double a, double b, double y) {
+    if (y == 0.0) return a / b;
+    const double q0 = a * y;
+    const double q1 = fma_d(fma_d(-b, q0, a), y, q0);
+    return fma_d(fma_d(-b, q1, a), y, q1);
+}
+
 CH_HD void distort(const DevCamera &c, double px, double py, double &ox, double &oy) {  // geometry.rs:325-330
-    double nx = (px - c.dist_center[0]) / c.dist_norm[0];
-    double ny = (py - c.dist_center[1]) / c.dist_norm[1];
+    double nx = div_by(px - c.dist_center[0], c.dist_norm[0], c.dist_norm_inverse[0]);
+    double ny = div_by(py - c.dist_center[1], c.dist_norm[1], c.dist_norm_inverse[1]);
     double dx, dy;
     distort_normalized(c.dist_coeffs, nx, ny, dx, dy);
     ox = dx * c.dist_norm[0] + c.dist_center[0];
@@ -442,10 +548,18 @@ CH_HD D3 along(D3 origin, D3 direction, double depth) {
     return {origin.x + direction.x * depth, origin.y + direction.y * depth, origin.z + direction.z * depth};
 }
 
+// A plane whose rows start 16-byte aligned: `pitch` floats apart, a multiple of 4.
+struct PaddedPlane {
+    const float *data;
+    int pitch;
+};
+
 // ---- device forms of the boundary types -------------------------------------------
 struct DevView {
     PlaneRef luma;
     const float4 *quads;  // bilinear neighbourhood (quad) plane of the luminance (targets only)
+    int quad_stride;      // of its rows, in quads (quad_index)
+    PaddedPlane rows_plane, columns_plane;  // the luminance and its transpose (targets only)
     WarpRef warp;
     int width, height;
     int has_camera, accepted;
@@ -467,6 +581,10 @@ inline void camera_from_abi(const chiaro_camera &a, DevCamera &c) {
     for (int i = 0; i < 2; ++i) {
         c.dist_center[i] = a.distortion_center[i];
         c.dist_norm[i] = a.distortion_normalization[i];
+    }
+    for (int i = 0; i < 2; ++i) {
+        const double norm = std::fabs(c.dist_norm[i]);
+        c.dist_norm_inverse[i] = norm >= 0x1p-500 && norm <= 0x1p500 ? 1.0 / c.dist_norm[i] : 0.0;
     }
     for (int i = 0; i < 5; ++i) c.dist_coeffs[i] = a.distortion_coeffs[i];
     memcpy(c.rotation_wc, a.rotation_wc, sizeof(c.rotation_wc));

@@ -105,6 +105,14 @@ __device__ __forceinline__ int list_items(const DecisionSlot &d, int count, bool
     return count + __popc(mask);
 }
 
+// The correlation of d's listed entry `at` (target v). The f64 form alone (zncc_any): a node
+// lists 24 or 32 items for one warp, so one item off the grid would cost the warp both loops.
+__device__ __forceinline__ bool decision_score(const DecisionParams &p, const DecisionSlot &d, const RefPatch &patch,
+                                               int at, int v, int taps, float &score) {
+    const double2 dd = d.disp[at];
+    return zncc_any<9>(p.views[p.targets[v]], d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y, score);
+}
+
 // Scores the pooled lists of the CTA's nodes (node k's count[k] entries of its
 // d.list / d.disp, node after node), so the lanes of all warps share the
 // correlations of one phase. Phase 1 items are (target, offset k < 5 or baseline
@@ -122,11 +130,8 @@ __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned ch
         const DecisionSlot d = carve_decision_slot(smem_raw + (size_t)k * slot_bytes, V, taps);
         const int item = d.list[at];
         const int v = shifts ? item >> 3 : item / 6;
-        const DevView &tv = p.views[p.targets[v]];
-        const double2 dd = d.disp[at];
         float score;
-        const bool ok = zncc_any(TargetRef{tv.luma, tv.quads}, d.gh + v * taps, d.box[v], d.wt, patches[k], taps,
-                                 dd.x, dd.y, score);
+        const bool ok = decision_score(p, d, patches[k], at, v, taps, score);
         const int kk = shifts ? 6 + (item & 7) : item - v * 6;
         if (ok)
             d.sc[v * 16 + kk] = score;
@@ -233,11 +238,8 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS) target_decision_kernel(De
         for (int j = lane; j < listed; j += 32) {
             const int item = d.list[j];
             const int v = item / 6, k = item - v * 6;
-            const DevView &tv = p.views[p.targets[v]];
-            const double2 dd = d.disp[j];
             float score;
-            if (zncc_any(TargetRef{tv.luma, tv.quads}, d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y,
-                         score))
+            if (decision_score(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + k] = score;
             else if (k < 5)
                 atomicOr(&d.flags[v], 1);
@@ -294,11 +296,8 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS) target_decision_kernel(De
         for (int j = lane; j < listed; j += 32) {
             const int item = d.list[j];
             const int v = item >> 3;
-            const DevView &tv = p.views[p.targets[v]];
-            const double2 dd = d.disp[j];
             float score;
-            if (zncc_any(TargetRef{tv.luma, tv.quads}, d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y,
-                         score))
+            if (decision_score(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + 6 + (item & 7)] = score;
             else
                 atomicOr(&d.flags[v], 1);

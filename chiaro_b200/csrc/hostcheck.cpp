@@ -55,6 +55,73 @@ uint64_t chiaro_hc_exp_mismatches(uint32_t lo, uint32_t hi, double scale, uint32
     return bad;
 }
 
+// grid_offset against the two-step f64 coordinate: random patches of positive half
+// positions and displacements (plain random ones, multiples of a power of two, and those
+// nudged by a few f64 ulps, where ties and their neighbours sit). Returns the mismatching
+// coordinates and counts the accepted patches.
+uint64_t chiaro_hc_grid_offset_mismatches(uint64_t patches, uint64_t seed, uint64_t *accepted) {
+    uint64_t state = seed * 0x9E3779B97F4A7C15ull + 1, bad = 0;
+    auto next = [&]() {  // xorshift64*
+        state ^= state >> 12;
+        state ^= state << 25;
+        state ^= state >> 27;
+        return state * 0x2545F4914F6CDD1Dull;
+    };
+    auto unit = [&]() { return (double)(next() >> 11) * 0x1p-53; };
+    *accepted = 0;
+    for (uint64_t i = 0; i < patches; ++i) {
+        const double centre = std::exp2(unit() * 13.0);
+        double d = (unit() * 2.0 - 1.0) * std::exp2(6.0 - unit() * (next() % 4 ? 4.0 : 60.0));
+        const int kind = (int)(next() % 4);
+        if (kind >= 2) {
+            const double grid = std::exp2(-(double)(next() % 28));
+            d = std::floor(d / grid) * grid;
+            if (kind == 3)
+                for (int k = (int)(next() % 4); k > 0; --k) d = std::nextafter(d, next() & 1 ? 100.0 : -100.0);
+        }
+        float g[9], x[9], lowest = INFINITY, g_lowest = INFINITY, highest = -INFINITY;
+        for (int t = 0; t < 9; ++t) {
+            g[t] = (float)(centre + (unit() * 2.0 - 1.0) * 12.0);
+            x[t] = (float)(((double)g[t] + d) - 0.25);
+            lowest = std::fmin(lowest, x[t]);
+            highest = std::fmax(highest, x[t]);
+            g_lowest = std::fmin(g_lowest, g[t]);
+        }
+        float e;
+        if (!(lowest >= 0.0f && highest < (float)(GRID_OFFSET_MAX_SIDE - 1)) || !grid_offset(d, g_lowest, e)) continue;
+        ++*accepted;
+        for (int t = 0; t < 9; ++t) {
+            const float y = g[t] + e;
+            bad += f2u(y) != f2u(x[t]);
+        }
+    }
+    return bad;
+}
+
+// div_by against the division, over random dividends and divisors of a normalisation's kind
+// and quotients next to a midpoint.
+uint64_t chiaro_hc_div_by_mismatches(uint64_t count, uint64_t seed) {
+    uint64_t state = seed * 0x9E3779B97F4A7C15ull + 1, bad = 0;
+    auto next = [&]() {
+        state ^= state >> 12;
+        state ^= state << 25;
+        state ^= state >> 27;
+        return state * 0x2545F4914F6CDD1Dull;
+    };
+    for (uint64_t i = 0; i < count; ++i) {
+        double b = u2d((next() & 0x000FFFFFFFFFFFFFull) | ((1023ull - 20 + next() % 41) << 52));
+        if (next() % 4 == 0) b = (double)(next() % 20000 + 1) * 0.8;
+        if (next() % 8 == 0) b = u2d(d2u(b) | 0x000FFFFFFFFFFFFFull);
+        double a = u2d((next() & 0x800FFFFFFFFFFFFFull) | ((1023ull - 20 + next() % 41) << 52));
+        if (next() % 2) {  // a quotient near the middle of two doubles
+            const double q = u2d((next() & 0x000FFFFFFFFFFFFFull) | (1023ull << 52));
+            a = std::fma(q, b, (next() & 1 ? 1 : -1) * b * 0x1p-53);
+        }
+        bad += d2u(div_by(a, b, 1.0 / b)) != d2u(a / b);
+    }
+    return bad;
+}
+
 // aggregate as the reference writes it (depth.rs:1761-1770): compaction, stable
 // insertion sort descending by f32::total_cmp, the sum of the best from -0.0.
 static bool aggregate_reference(const float *in, int n, int minimum_support, int best_view_count, float &out) {

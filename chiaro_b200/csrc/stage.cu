@@ -213,8 +213,9 @@ void set_smem_limits() {
     CK(cudaFuncSetAttribute(cost_volume_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(cost_volume_kernel<160>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(cost_volume_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(direct_depth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(direct_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false>,
+                        direct_wide_kernel<true>})
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(target_decision_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(target_decision_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(align_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -222,7 +223,7 @@ void set_smem_limits() {
 }
 
 // ---- cost-volume launch shapes (the autotuner) -----------------------------------------
-typedef void (*CostKernel)(CostParams);
+typedef void (*CostKernel)(CostParams, int);
 
 CostKernel cost_kernel_for(int threads) {
     switch (threads) {
@@ -234,13 +235,82 @@ CostKernel cost_kernel_for(int threads) {
     }
 }
 
-// Launch build_cost_volume over n_rows node CTAs. With autotuning on, the first launch of a
+// The tile, the region buffer and each target's axis and passes for a cost-volume launch.
+// A target's epipolar segment is taken at the reference's centre: its direction decides
+// whether samples are stored by rows or by columns, and its extent how many parts the labels
+// are scored in, so that a part's samples fit the region buffer. Elsewhere in the image the
+// segment differs a little; a tile whose samples do not fit gathers from the quad plane.
+// 48 rows: 4160x3120, 129 labels took 9.96 / 9.97 / 9.24 / 9.71 ms at 32 / 40 / 48 / 56 rows
+// (fewer rows mean more parts, more rows fewer CTAs an SM). Tiles, cost volume of 2080x1560 with
+// 65 labels, two targets, at 1 / 2 / 4 / 8 nodes: 3.83 / 2.93 / 2.26 / 2.08 ms; 1567x1173 with 193
+// labels, three targets: 1.86 / 1.58 / 1.47 / 1.52 ms; 1040x780 with 17 labels, four targets: 0.64 /
+// 0.45 / 0.33 / 0.31 ms. Eight nodes pay for few labels, and a grid of few nodes takes smaller
+// tiles so that every SM has several (320x240, 25 labels: 0.127 ms at 2 nodes, 0.129 at 4 and 8).
+constexpr int COST_REGION_ROWS = 48;
+
+void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_rows, int sm_count) {
+    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
+    p.region_rows = COST_REGION_ROWS;
+    p.one = 1.0f;
+    const int shapes[4][2] = {{4, 2}, {2, 2}, {2, 1}, {1, 1}};
+    for (const auto &shape : shapes) {
+        const int nodes = shape[0] * shape[1];
+        p.tile_w = p.node_list ? nodes : shape[0];
+        p.tile_h = p.node_list ? 1 : shape[1];
+        if (nodes == 8 && (p.slots > 80 || n_rows < (size_t)16 * nodes * sm_count) && p.slots > 32)
+            continue;  // four nodes fill the CTA's threads
+        if (n_rows < (size_t)nodes * 4 * sm_count) continue;  // a small grid: more CTAs instead
+        if (tile_smem_bytes(nodes, taps, p.slots, p.region_rows) <= 56 * 1024) break;
+    }
+    const DevView &rv = views[p.reference];
+    for (int v = 0; v < p.n_targets; ++v) {
+        const DevView &tv = views[p.targets[v]];
+        p.transposed[v] = 0;
+        p.passes[v] = 1;
+        D3 origin, direction;
+        double x0, y0, x1, y1;
+        pixel_to_ray(rv.cam, rv.width * 0.5, rv.height * 0.5, origin, direction);
+        if (!project(tv.cam, along(origin, direction, INFINITY_DEPTH), x0, y0) ||
+            !project(tv.cam, along(origin, direction, p.near_depth), x1, y1))
+            continue;
+        const double dx = std::fabs(x1 - x0) * 0.5, dy = std::fabs(y1 - y0) * 0.5;  // samples
+        if (!(std::isfinite(dx) && std::isfinite(dy))) continue;
+        p.transposed[v] = dy > dx;
+        // the share of the segment that the scored labels cover, and the room for it beside the
+        // patch, the tile's nodes, the bilinear neighbour, alignment and the warp's own bending
+        const double share = p.band_first ? (double)p.slots / p.labels : 1.0;
+        const double fixed = 2 * p.radius + 8, step = p.step * 0.5;
+        const double wide = (p.transposed[v] ? p.tile_h : p.tile_w) - 1, high = (p.transposed[v] ? p.tile_w : p.tile_h) - 1;
+        const double room_wide = std::max(REGION_PITCH - 3 - fixed - wide * step, 8.0);
+        const double room_high = std::max(p.region_rows - fixed - high * step, 8.0);
+        // 64 samples are the reach of a hypothesis (depth.rs:1611-1613)
+        const double longest = std::max(dx, dy) * share;
+        const double parts_wide = std::min(longest, 64.0) > room_wide ? longest / room_wide : 1.0;
+        const double slope = std::min(dx, dy) / std::max(std::max(dx, dy), 1e-9);
+        const double parts_high = std::min(longest, 64.0) * slope > room_high ? longest * slope / room_high : 1.0;
+        p.passes[v] = (unsigned char)std::max(1.0, std::min({std::ceil(std::max(parts_wide, parts_high)), 8.0,
+                                                             (double)p.slots}));
+    }
+}
+
+// Launch build_cost_volume over n_rows nodes. With autotuning on, the first launch of a
 // (targets, labels scored, radius) bucket large enough to time (at least 4096 nodes, outside
 // any stream capture) runs every shape twice and keeps the fastest second run for the
 // context's later launches; every shape writes the same bits, and the last launch below
 // writes the outputs again.
-void launch_cost(chiaro_depth_ctx *ctx, const CostParams &p, size_t n_rows, size_t smem) {
+void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView> &views, size_t n_rows,
+                 size_t path_floats) {
     cudaStream_t s = ctx->stream;
+    plan_cost_tiles(p, views, n_rows, ctx->sm_count);
+    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1), nodes = p.tile_w * p.tile_h;
+    const size_t smem = tile_smem_bytes(nodes, taps, p.slots, p.region_rows);
+    const unsigned blocks = (unsigned)(p.node_list ? div_ceil(n_rows, nodes)
+                                                   : div_ceil(p.columns, p.tile_w) * div_ceil(p.rows, p.tile_h));
+    // the launch's scratch shares the SGM's path buffers, which are free until the volume is done
+    const size_t items = (size_t)blocks * nodes * p.slots;
+    float *scratch = dbuf<float>(ctx, "sgm_paths", std::max(items * (4 + p.n_targets), path_floats));
+    p.places = reinterpret_cast<double2 *>(scratch);
+    p.view_scores = scratch + 4 * items;
     const uint64_t key = ((uint64_t)p.n_targets << 24) | ((uint64_t)p.slots << 8) | (uint64_t)p.radius;
     int threads = ctx->autotune > 1 ? ctx->autotune : COST_THREADS;
     auto it = ctx->cost_tuning.find(key);
@@ -259,7 +329,7 @@ void launch_cost(chiaro_depth_ctx *ctx, const CostParams &p, size_t n_rows, size
             float ms = 0.0f;
             for (int rep = 0; rep < 2; ++rep) {
                 CK(cudaEventRecord(e0, s));
-                cost_kernel_for(t)<<<(unsigned)n_rows, t, smem, s>>>(p);
+                cost_kernel_for(t)<<<blocks, t, smem, s>>>(p, (int)n_rows);
                 CK(cudaGetLastError());
                 CK(cudaEventRecord(e1, s));
                 CK(cudaEventSynchronize(e1));
@@ -274,24 +344,66 @@ void launch_cost(chiaro_depth_ctx *ctx, const CostParams &p, size_t n_rows, size
         cudaEventDestroy(e1);
         ctx->cost_tuning[key] = threads;
     }
-    cost_kernel_for(threads)<<<(unsigned)n_rows, threads, smem, s>>>(p);
+    cost_kernel_for(threads)<<<blocks, threads, smem, s>>>(p, (int)n_rows);
     CK(cudaGetLastError());
 }
 
-// Per (node, target) geometry records of a step-spaced grid.
+// Per (node, target) geometry records of one or two step-spaced grids.
 void launch_geometry(chiaro_depth_ctx *ctx, const DevView *d_views, int reference, const std::vector<int> &targets,
-                     size_t columns, size_t rows, size_t step, GeomRec *out) {
+                     const std::vector<GeometryGrid> &grids) {
     if (targets.empty()) return;
     GeometryParams p{};
     p.views = d_views;
     p.reference = reference;
     p.n_targets = (int)targets.size();
     for (size_t v = 0; v < targets.size(); ++v) p.targets[v] = targets[v];
-    p.columns = (int)columns;
-    p.rows = (int)rows;
-    p.step = (int)step;
-    p.out = out;
-    view_geometry_kernel<<<blocks_for(columns * rows * targets.size(), 128), 128, 0, ctx->stream>>>(p);
+    size_t most = 0;
+    for (size_t i = 0; i < grids.size(); ++i) {
+        p.grids[i] = grids[i];
+        most = std::max(most, (size_t)grids[i].columns * grids[i].rows);
+    }
+    view_geometry_kernel<<<dim3(blocks_for(most * targets.size(), 128), (unsigned)grids.size()), 128, 0, ctx->stream>>>(p);
+    CK(cudaGetLastError());
+}
+
+// The buffers of a target's planes for the correlations: quads, padded rows, padded columns.
+void sample_planes(chiaro_depth_ctx *ctx, int t, DevView &v) {
+    const PlaneRef &lp = v.luma;
+    const std::string name = std::to_string(t);
+    v.quad_stride = quad_stride(lp.width);
+    v.quads = dbuf<float4>(ctx, "quads" + name, quad_count(lp.width, lp.height));
+    v.rows_plane.pitch = (lp.width + 3) / 4 * 4;
+    v.rows_plane.data = dbuf<float>(ctx, "rows" + name, (size_t)v.rows_plane.pitch * lp.height);
+    v.columns_plane.pitch = (lp.height + 3) / 4 * 4;
+    v.columns_plane.data = dbuf<float>(ctx, "columns" + name, (size_t)v.columns_plane.pitch * lp.width);
+}
+
+void launch_sample_planes(chiaro_depth_ctx *ctx, const DevView *d_views, const std::vector<DevView> &views,
+                          const std::vector<int> &targets) {
+    if (targets.empty()) return;
+    PlanesParams p{};
+    p.views = d_views;
+    size_t most = 0;
+    for (size_t v = 0; v < targets.size(); ++v) {
+        const PlaneRef &lp = views[targets[v]].luma;
+        p.targets[v] = targets[v];
+        most = std::max(most, div_ceil(lp.width, 32) * div_ceil(lp.height, 32));
+    }
+    sample_planes_kernel<<<dim3((unsigned)most, (unsigned)targets.size()), dim3(32, 8), 0, ctx->stream>>>(p);
+    CK(cudaGetLastError());
+}
+
+// The reference patches of one or two grids' nodes (patch_sums_kernel).
+void launch_patches(chiaro_depth_ctx *ctx, const DevView *d_views, int reference, const std::vector<PatchGrid> &grids) {
+    PatchParams p{};
+    p.views = d_views;
+    p.reference = reference;
+    size_t most = 0;
+    for (size_t i = 0; i < grids.size(); ++i) {
+        p.grids[i] = grids[i];
+        most = std::max(most, (size_t)grids[i].columns * grids[i].rows);
+    }
+    patch_sums_kernel<<<dim3(blocks_for(most, 256), (unsigned)grids.size()), 256, 0, ctx->stream>>>(p);
     CK(cudaGetLastError());
 }
 
@@ -1048,6 +1160,8 @@ struct CoarseGrid {
     float *spatial;
     GeomRec *geometry;
     TapLattice lattice;
+    RefPatch *patches;
+    std::vector<DevView> h_views;
     DevView *views;
 };
 
@@ -1074,6 +1188,8 @@ void coarse_cost(chiaro_depth_ctx *ctx, const CoarseGrid &g, int reference, cons
     }
     p.node_list = node_list;
     p.label_depth = g.labels;
+    p.near_depth = o.near_depth;
+    p.patches = g.patches;
     p.spatial = g.spatial;
     p.radius = (int)o.patch_radius;
     p.lattice = g.lattice;
@@ -1084,10 +1200,9 @@ void coarse_cost(chiaro_depth_ctx *ctx, const CoarseGrid &g, int reference, cons
     p.guidance = guidance;
     p.tested = tested;
     const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
-    const size_t smem = node_smem_bytes(g.V, taps, slots);
-    if ((size_t)g.V * slots > 65535 || smem > 200 * 1024)
+    if ((size_t)g.V * slots > 65535 || node_smem_bytes(g.V, taps, slots) > 200 * 1024)
         throw CudaError{cudaErrorInvalidValue, "cost volume: targets x labels exceed the node CTA's shared memory"};
-    launch_cost(ctx, p, n_rows, smem);
+    launch_cost(ctx, p, g.h_views, n_rows, 0);
 }
 
 // The coarse search of the stage's reference grid (depth.rs:1187-1467 up to the winner):
@@ -1120,11 +1235,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     g.spatial = dbuf<float>(ctx, "coarse.spatial", sp.size());
     upload(ctx, g.labels, labels.data(), D);
     upload(ctx, g.spatial, sp.data(), sp.size());
-    for (int t : g.targets) {
-        const PlaneRef &lp = h_views[t].luma;
-        h_views[t].quads = dbuf<float4>(ctx, "quads" + std::to_string(t),
-                                        (size_t)quad_pair_stride(lp.width) * ((lp.height + 1) / 2));
-    }
+    for (int t : g.targets) sample_planes(ctx, t, h_views[t]);
     g.views = dbuf<DevView>(ctx, "coarse.views", n_views);
     upload(ctx, g.views, h_views.data(), n_views);
     g.geometry = dbuf<GeomRec>(ctx, "coarse_geometry", N * std::max(g.V, 1));
@@ -1135,7 +1246,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         g.lattice.planes = dbuf<float2>(ctx, "coarse.lattice", (size_t)(g.V + 1) * g.lattice.columns * g.lattice.rows);
     }
     CK(cudaEventRecord(ctx->events[0], s));
-    launch_geometry(ctx, g.views, reference, g.targets, g.columns, g.rows, g.step, g.geometry);
+    launch_geometry(ctx, g.views, reference, g.targets, {{g.columns, g.rows, g.step, g.geometry}});
     if (g.lattice.planes) {
         LatticeParams p{};
         p.views = g.views;
@@ -1149,12 +1260,10 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         tap_lattice_kernel<<<blocks_for((size_t)g.lattice.columns * g.lattice.rows, 256), 256, 0, s>>>(p);
         CK(cudaGetLastError());
     }
-    for (int t : g.targets) {
-        const PlaneRef &lp = h_views[t].luma;
-        quad_plane_kernel<<<blocks_for((size_t)lp.width * lp.height, 256), 256, 0, s>>>(
-            lp.data, lp.width, lp.height, quad_pair_stride(lp.width), const_cast<float4 *>(h_views[t].quads));
-        CK(cudaGetLastError());
-    }
+    launch_sample_planes(ctx, g.views, h_views, g.targets);
+    g.h_views = h_views;
+    g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
+    launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
     CK(cudaEventRecord(ctx->events[1], s));
     uint8_t *tested = dbuf<uint8_t>(ctx, "coarse.tested", N);
     float *guidance = dbuf<float>(ctx, "coarse.guidance", N);
@@ -1561,11 +1670,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     upload(ctx, d_sp_wide, sp_wide.data(), sp_wide.size());
     upload(ctx, d_sp25, spatial25.data(), 25);
     // the quad planes' buffers and the views that point at them, before any launch
-    for (int t : targets) {
-        const PlaneRef &lp = h_views[t].luma;
-        h_views[t].quads = dbuf<float4>(ctx, "quads" + std::to_string(t),
-                                        (size_t)quad_pair_stride(lp.width) * ((lp.height + 1) / 2));
-    }
+    for (int t : targets) sample_planes(ctx, t, h_views[t]);
     upload(ctx, d_views, h_views.data(), h_views.size());
     GeomRec *coarse_geometry = dbuf<GeomRec>(ctx, "coarse_geometry", N * std::max(V, 1));
     GeomRec *fine_geometry = dbuf<GeomRec>(ctx, "fine_geometry", M * std::max(V, 1));
@@ -1587,9 +1692,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         lattice.rows = (int)(extent_y / 2 + 2 * (size_t)lattice.margin + 1);
         lattice.planes = dbuf<float2>(ctx, "tap_lattice", (size_t)(V + 1) * lattice.columns * lattice.rows);
     }
-    // quad planes 1 per target, tap lattice 1, geometry 2, cost 1, SGM 2, select 1, completion, direct 2, filters 6, stats 2,
-    // decisions 1 + 3 per target, map 1
-    ctx->launches = V + (V > 0 ? 2 : 0) + (lattice.planes ? 1 : 0) + 1 + 2 + 1 + (int)o.completion_iterations + 3 + 6 +
+    // sample planes and geometry 1 each, tap lattice 1, patches 1, cost 1, SGM 2, select 1, completion, direct 2,
+    // filters 6, stats 2, decisions 1 + 3 per target, map 1
+    ctx->launches = (V > 0 ? 2 : 0) + (lattice.planes ? 1 : 0) + 1 + 1 + 2 + 1 + (int)o.completion_iterations + 2 + 6 +
                     2 + (V > 0 ? 1 + 3 * V : 0) + 1;
     // the whole-stage graph (device-buffer calls only)
     ctx->stage_graph_state = 0;
@@ -1626,9 +1731,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     record_event(ctx->events[0], s, capturing);
     // per (node, target) geometry of both grids: cameras and warps only, so it runs
     // while the luminance planes are still arriving
-    launch_geometry(ctx, d_views, reference, targets, g.coarse_columns, g.coarse_rows, g.coarse_step,
-                    coarse_geometry);
-    launch_geometry(ctx, d_views, reference, targets, g.columns, g.rows, g.step, fine_geometry);
+    launch_geometry(ctx, d_views, reference, targets,
+                    {{(int)g.columns, (int)g.rows, (int)g.step, fine_geometry},
+                     {(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, coarse_geometry}});
     // the reference's plane goes up first: the tap lattice and the fine reference patches
     // need only it (and the warps), so they run while the targets' planes arrive
     const bool host_planes = host && !host->planes.empty();
@@ -1660,29 +1765,15 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     // each fine node's reference patch at the direct radius, read by the direct pass and,
     // at the same radius, by the decisions
     RefPatch *fine_patches = dbuf<RefPatch>(ctx, "fine_patches", M);
-    {
-        PatchParams pp{};
-        pp.views = d_views;
-        pp.reference = reference;
-        pp.columns = (int)g.columns;
-        pp.rows = (int)g.rows;
-        pp.step = (int)g.step;
-        pp.radius = direct_radius;
-        pp.spatial = d_sp_direct;
-        if (fine_lattice) pp.lattice = lattice;
-        pp.out = fine_patches;
-        patch_sums_kernel<<<blocks_for(M, 256), 256, 0, s>>>(pp);
-        CK(cudaGetLastError());
-    }
+    RefPatch *coarse_patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
+    launch_patches(ctx, d_views, reference,
+                   {{(int)g.columns, (int)g.rows, (int)g.step, direct_radius, d_sp_direct,
+                     fine_lattice ? lattice : TapLattice{}, fine_patches},
+                    {(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, radius, d_sp,
+                     coarse_lattice ? lattice : TapLattice{}, coarse_patches}});
     if (host_planes) CK(cudaStreamWaitEvent(s, ctx->planes_ready, 0));
     // quad planes of the target luminance for the fast ZNCC path
-    for (int t : targets) {
-        const PlaneRef &lp = h_views[t].luma;
-        size_t n = (size_t)lp.width * lp.height;
-        quad_plane_kernel<<<blocks_for(n, 256), 256, 0, s>>>(lp.data, lp.width, lp.height, quad_pair_stride(lp.width),
-                                                             const_cast<float4 *>(h_views[t].quads));
-        CK(cudaGetLastError());
-    }
+    launch_sample_planes(ctx, d_views, h_views, targets);
     // ---- cost volume
     float *scores = dbuf<float>(ctx, "scores", N * D);
     float *costs = dbuf<float>(ctx, "costs", N * D);
@@ -1702,6 +1793,8 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         p.labels = D;
         p.slots = D;
         p.label_depth = d_labels;
+        p.near_depth = o.near_depth;
+        p.patches = coarse_patches;
         p.spatial = d_sp;
         p.radius = radius;
         if (coarse_lattice) p.lattice = lattice;
@@ -1712,10 +1805,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         p.guidance = guidance;
         p.tested = tested;
         int taps = (2 * radius + 1) * (2 * radius + 1);
-        const size_t smem = node_smem_bytes(V, taps, D);
-        if ((size_t)V * D > 65535 || smem > 200 * 1024)
+        if ((size_t)V * D > 65535 || node_smem_bytes(V, taps, D) > 200 * 1024)
             throw CudaError{cudaErrorInvalidValue, "cost volume: targets x labels exceed the node CTA's shared memory"};
-        launch_cost(ctx, p, N, smem);
+        launch_cost(ctx, p, h_views, N, 8 * ((N * D + 63) / 64 * 64));
     }
     record_event(ctx->events[1], s, capturing);
     // ---- SGM
@@ -1809,14 +1901,18 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         const size_t slot = direct_slot_bytes<float2>(V, taps), wide_slot = direct_slot_bytes<float2>(V, wide_taps);
         if (slot > 200 * 1024 || wide_slot > 200 * 1024)
             throw CudaError{cudaErrorInvalidValue, "direct pass shared memory exceeds 200 KiB"};
-        p.nodes_per_cta = warps_per_cta(direct_depth_kernel, slot, 8);
-        direct_depth_kernel<<<blocks_for(M, p.nodes_per_cta), 32 * p.nodes_per_cta, p.nodes_per_cta * slot, s>>>(p);
+        bool grid = true;  // see DIRECT_GRID_SIDE
+        for (int t : targets) grid = grid && std::max(h_views[t].luma.width, h_views[t].luma.height) >= DIRECT_GRID_SIDE;
+        const auto direct_kernel = grid ? direct_depth_kernel<true> : direct_depth_kernel<false>;
+        const auto wide_kernel = grid ? direct_wide_kernel<true> : direct_wide_kernel<false>;
+        p.nodes_per_cta = warps_per_cta(direct_kernel, slot, 8);
+        direct_kernel<<<blocks_for(M, p.nodes_per_cta), 32 * p.nodes_per_cta, p.nodes_per_cta * slot, s>>>(p);
         CK(cudaGetLastError());
-        const int wide_warps = warps_per_cta(direct_wide_kernel, wide_slot, 8);
+        const int wide_warps = warps_per_cta(wide_kernel, wide_slot, 8);
         int wide_blocks = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_blocks, direct_wide_kernel, 32 * wide_warps,
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_blocks, wide_kernel, 32 * wide_warps,
                                                          wide_warps * wide_slot));
-        direct_wide_kernel<<<ctx->sm_count * std::max(1, wide_blocks), 32 * wide_warps, wide_warps * wide_slot,
+        wide_kernel<<<ctx->sm_count * std::max(1, wide_blocks), 32 * wide_warps, wide_warps * wide_slot,
                              s>>>(p);
         CK(cudaGetLastError());
     }

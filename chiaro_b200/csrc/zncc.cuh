@@ -34,7 +34,7 @@ struct ViewGeom {
 };
 
 struct TapBox {
-    double xmin, xmax, ymin, ymax;  // of g/2 over the taps
+    float xmin, xmax, ymin, ymax;  // of g/2 over the taps
 };
 
 __device__ __forceinline__ void tap_offset(int t, int radius, int &dx, int &dy) {
@@ -50,43 +50,70 @@ __device__ __forceinline__ void tap_offset(int t, int radius, const SmallDiv &si
     dx = t - row * (int)side.d - radius;
 }
 
-// Tap positions are kept either as g/2 in f64 (double2: one 16-byte load per
-// tap on the fast path) or as g in f32 (float2: half the shared memory, halved
-// to f64 at use). g is f32 and halving is exact in f64, so both give the same
-// bits everywhere.
-__device__ __forceinline__ double2 tap_half(const double2 &v) { return v; }
-__device__ __forceinline__ double2 tap_half(const float2 &v) {
-    return make_double2((double)v.x * 0.5, (double)v.y * 0.5);
+// A tap's position in a target is kept as g/2: in f32 (g is f32 and halving is exact, a
+// subnormal g apart, which no sample coordinate can tell from 0), or, for the f64 form alone,
+// in f64, which spares it a conversion per coordinate. The weights (w, w r) lie apart, once per
+// node.
+template <typename Half>
+struct Tap {
+    Half half;       // g/2
+    float2 weights;  // (w, w r)
+};
+template <typename Half>
+__device__ __forceinline__ Tap<Half> load_tap(const Half *taps, const float2 *wt, int t) {
+    return {taps[t], wt[t]};
 }
-__device__ __forceinline__ float2 tap_g(const double2 &v) {
-    return make_float2((float)(v.x * 2.0), (float)(v.y * 2.0));
-}
-__device__ __forceinline__ float2 tap_g(const float2 &v) { return v; }
 __device__ __forceinline__ void store_tap(double2 &d, float qx, float qy) {
     d = make_double2((double)qx * 0.5, (double)qy * 0.5);
 }
-__device__ __forceinline__ void store_tap(float2 &d, float qx, float qy) { d = make_float2(qx, qy); }
+__device__ __forceinline__ void store_tap(float2 &d, float qx, float qy) { d = make_float2(qx * 0.5f, qy * 0.5f); }
+
+// The taps of a patch in pairs, for packed arithmetic over both: half = (g/2 x, g/2 x', g/2 y,
+// g/2 y') per target, weight = (w, w', w r, w' r'). A patch has an odd number of taps: the last
+// pair's second half is unused.
+struct PairedTaps {
+    const float4 *half, *weight;
+};
+__device__ __forceinline__ Tap<float2> load_tap(const PairedTaps &taps, const float2 *, int t) {
+    const float *g = reinterpret_cast<const float *>(taps.half + (t >> 1)) + (t & 1);
+    const float *w = reinterpret_cast<const float *>(taps.weight + (t >> 1)) + (t & 1);
+    return {make_float2(g[0], g[2]), make_float2(w[0], w[2])};
+}
+
+__device__ __forceinline__ float warp_min_f(float v) {
+    float r;
+    asm volatile("redux.sync.min.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(0xffffffffu));
+    return r;
+}
+__device__ __forceinline__ float warp_max_f(float v) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, %2;" : "=f"(r) : "f"(v), "r"(0xffffffffu));
+    return r;
+}
+// The box of every lane's box.
+__device__ __forceinline__ TapBox warp_tap_box(const TapBox &b) {
+    return {warp_min_f(b.xmin), warp_max_f(b.xmax), warp_min_f(b.ymin), warp_max_f(b.ymax)};
+}
 
 // Bounding box of g/2 over one target's taps, computed by an aligned group of
 // eight lanes (min and max are exact, so the reduction order does not matter).
 // Every lane of the warp calls it; the groups reduce with shuffles.
 template <typename TapT>
 __device__ inline TapBox group8_tap_box(const TapT *gh, int taps) {
-    const double2 g0 = tap_half(gh[0]);
-    TapBox b{g0.x, g0.x, g0.y, g0.y};
+    TapBox b{(float)gh[0].x, (float)gh[0].x, (float)gh[0].y, (float)gh[0].y};
     for (int t = threadIdx.x & 7; t < taps; t += 8) {
-        const double2 g = tap_half(gh[t]);
-        b.xmin = fmin(b.xmin, g.x);
-        b.xmax = fmax(b.xmax, g.x);
-        b.ymin = fmin(b.ymin, g.y);
-        b.ymax = fmax(b.ymax, g.y);
+        const float gx = (float)gh[t].x, gy = (float)gh[t].y;
+        b.xmin = fminf(b.xmin, gx);
+        b.xmax = fmaxf(b.xmax, gx);
+        b.ymin = fminf(b.ymin, gy);
+        b.ymax = fmaxf(b.ymax, gy);
     }
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) {
-        b.xmin = fmin(b.xmin, __shfl_xor_sync(0xffffffffu, b.xmin, off));
-        b.xmax = fmax(b.xmax, __shfl_xor_sync(0xffffffffu, b.xmax, off));
-        b.ymin = fmin(b.ymin, __shfl_xor_sync(0xffffffffu, b.ymin, off));
-        b.ymax = fmax(b.ymax, __shfl_xor_sync(0xffffffffu, b.ymax, off));
+        b.xmin = fminf(b.xmin, __shfl_xor_sync(0xffffffffu, b.xmin, off));
+        b.xmax = fmaxf(b.xmax, __shfl_xor_sync(0xffffffffu, b.xmax, off));
+        b.ymin = fminf(b.ymin, __shfl_xor_sync(0xffffffffu, b.ymin, off));
+        b.ymax = fmaxf(b.ymax, __shfl_xor_sync(0xffffffffu, b.ymax, off));
     }
     return b;
 }
@@ -95,15 +122,6 @@ __device__ inline TapBox group8_tap_box(const TapT *gh, int taps) {
 // patch sums add w, w r and (w r) r tap by tap).
 __device__ inline float sequential_sum(const float *a, int stride, int taps) {
     float sum = 0.0f;
-    for (int t = 0; t < taps; ++t) sum += a[t * stride];
-    return sum;
-}
-
-// The same sum unrolled by nine (the same order of additions), for the cost volume, whose
-// three lanes summing hold up the node's CTA.
-__device__ inline float sequential_sum_unrolled(const float *a, int stride, int taps) {
-    float sum = 0.0f;
-#pragma unroll 9
     for (int t = 0; t < taps; ++t) sum += a[t * stride];
     return sum;
 }
@@ -194,29 +212,29 @@ __device__ inline unsigned warp_stage_patch(const DevView *views, int reference,
         int dx, dy;
         tap_offset(t, radius, dx, dy);
         float value = 0.0f;
+        const double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
+        const size_t at = at0 + (ptrdiff_t)dy * lattice.columns + dx;
         if (lattice.planes) {
-            const size_t at = at0 + (ptrdiff_t)dy * lattice.columns + dx;
             const float2 r = __ldg(lattice.planes + at);
             value = r.x;
             sampled &= r.y != 0.0f;
-            for (int v = 0; v < V; ++v) {
-                const float2 q = __ldg(lattice.planes + (size_t)(v + 1) * lattice.plane_size() + at);
-                if (q.x != q.x) undefined |= 1u << v;
-                store_tap(gh[v * taps + t], q.x, q.y);
-            }
         } else {
-            double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
             sampled &= plane_sample(rv.luma, (float)((px - 0.5) * 0.5), (float)((py - 0.5) * 0.5), value);
-            for (int v = 0; v < V; ++v) {
-                float qx = 0.0f, qy = 0.0f;
-                if (!warp_map(views[targets[v]].warp, (float)px, (float)py, qx, qy)) undefined |= 1u << v;
-                store_tap(gh[v * taps + t], qx, qy);
-            }
         }
-        float weight = spatial[t] * exp_f32(-1.2f * fabsf(value - centre));
-        float weighted = weight * value;
-        wt[t] = make_float2(weight, weighted);
-        rr[t] = weighted * value;
+        const float weight = spatial[t] * exp_f32(-1.2f * fabsf(value - centre));
+        const float2 weights = make_float2(weight, weight * value);
+        wt[t] = weights;
+        if (!pre) rr[t] = weights.y * value;
+        for (int v = 0; v < V; ++v) {
+            float2 q = make_float2(0.0f, 0.0f);
+            if (lattice.planes) {
+                q = __ldg(lattice.planes + (size_t)(v + 1) * lattice.plane_size() + at);
+                if (q.x != q.x) undefined |= 1u << v;
+            } else if (!warp_map(views[targets[v]].warp, (float)px, (float)py, q.x, q.y)) {
+                undefined |= 1u << v;
+            }
+            store_tap(gh[v * taps + t], q.x, q.y);
+        }
     }
     undefined = __reduce_or_sync(full, undefined);
     sampled = __all_sync(full, sampled);
@@ -250,20 +268,25 @@ __device__ inline unsigned warp_stage_patch(const DevView *views, int reference,
 // whether the centre and every tap were sampled), with the same expressions in the same
 // order, so the same bits. The direct pass and the decisions read it instead of summing 81
 // or more taps in three lanes of a warp.
-struct PatchParams {
-    const DevView *views;
-    int reference;
+// Grid row y of the launch works on grid y (the fine and the coarse one).
+struct PatchGrid {
     int columns, rows, step, radius;
     const float *spatial;
     TapLattice lattice;  // of this grid, or planes == nullptr
     RefPatch *out;
 };
+struct PatchParams {
+    const DevView *views;
+    int reference;
+    PatchGrid grids[2];
+};
 
-__global__ void __launch_bounds__(256) patch_sums_kernel(PatchParams p) {
+__global__ void __launch_bounds__(256) patch_sums_kernel(PatchParams params) {
+    const PatchGrid &p = params.grids[blockIdx.y];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= (long)p.columns * p.rows) return;
     const double cx = (double)((int)(i % p.columns) * p.step), cy = (double)((int)(i / p.columns) * p.step);
-    const DevView &rv = p.views[p.reference];
+    const DevView &rv = params.views[params.reference];
     const TapLattice &lattice = p.lattice;
     const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
     float centre = 0.0f;
@@ -360,22 +383,28 @@ __device__ __forceinline__ void geom_from_rec(const GeomRec &rec, const D3 &orig
 }
 
 // One thread per (node, target) of a step-spaced grid: the label-independent
-// part of map_at_depth (depth.rs:1745-1756).
+// part of map_at_depth (depth.rs:1745-1756). Grid row y of the launch works on grid y (the
+// coarse and the fine one).
+struct GeometryGrid {
+    int columns, rows, step;
+    GeomRec *out;  // [node][target]
+};
 struct GeometryParams {
     const DevView *views;
     int reference, n_targets;
     int targets[MAX_VIEWS];
-    int columns, rows, step;
-    GeomRec *out;  // [node][target]
+    GeometryGrid grids[2];
 };
 
-__global__ void __launch_bounds__(128) view_geometry_kernel(GeometryParams p) {
+__global__ void __launch_bounds__(128) view_geometry_kernel(GeometryParams params) {
+    const GeometryParams &p = params;
+    const GeometryGrid &grid = p.grids[blockIdx.y];
     long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    long total = (long)p.columns * p.rows * p.n_targets;
+    long total = (long)grid.columns * grid.rows * p.n_targets;
     if (i >= total) return;
     int v = (int)(i % p.n_targets);
     int node = (int)(i / p.n_targets);
-    double cx = (double)((node % p.columns) * p.step), cy = (double)((node / p.columns) * p.step);
+    double cx = (double)((node % grid.columns) * grid.step), cy = (double)((node / grid.columns) * grid.step);
     const DevView &tv = p.views[p.targets[v]];
     ViewGeom g;
     view_geometry(p.views[p.reference].cam, tv.cam, tv.warp, cx, cy, g);
@@ -385,7 +414,7 @@ __global__ void __launch_bounds__(128) view_geometry_kernel(GeometryParams p) {
     rec.dx = g.ray_ok ? g.dx : NAN;
     rec.dy = g.ray_ok ? g.dy : NAN;
     rec.dz = g.ray_ok ? g.dz : NAN;
-    p.out[i] = rec;
+    grid.out[i] = rec;
 }
 
 // map_at_depth's last step and score_one_view's displacement check: the
@@ -405,16 +434,16 @@ __device__ __forceinline__ bool depth_delta(const DevCamera &tc, const ViewGeom 
 // Hypothesis-dependent part of warped_patch_zncc: sample the target at every
 // tap shifted by (ddx, ddy) and finish the correlation. False for None.
 template <typename TapT>
-__device__ __forceinline__ bool zncc_score(const PlaneRef &target, const TapT *gh, const float2 *wt,
+__device__ __forceinline__ bool zncc_score(const PlaneRef &target, TapT gh, const float2 *wt,
                                            const RefPatch &patch, int taps, double ddx, double ddy, float &score) {
     float st = 0.0f, stt = 0.0f, srt = 0.0f;
     for (int t = 0; t < taps; ++t) {
-        const float2 g = tap_g(gh[t]);  // the tap's global-warp position
-        double qx = (double)g.x + ddx;
-        double qy = (double)g.y + ddy;
+        const auto tap = load_tap(gh, wt, t);
+        double qx = (double)tap.half.x * 2.0 + ddx;
+        double qy = (double)tap.half.y * 2.0 + ddy;
         float tv;
         if (!plane_sample(target, (float)((qx - 0.5) * 0.5), (float)((qy - 0.5) * 0.5), tv)) return false;
-        const float2 weights = wt[t];
+        const float2 weights = tap.weights;
         float wv = weights.x * tv;
         st += wv;
         stt += wv * tv;
@@ -428,17 +457,19 @@ __device__ __forceinline__ bool zncc_score(const PlaneRef &target, const TapT *g
     return true;
 }
 
-// ---- fast path ---------------------------------------------------------------------
+// ---- fast paths --------------------------------------------------------------------
 // The reference computes each target sample coordinate as
 //   x = (f32)(((f64)g + d - 0.5) * 0.5)
 // with two f64 roundings. Multiplying by 0.5 is exact and commutes with
 // rounding, so the same bits come from x = (f32)((g/2 + d/2) - 0.25), where g/2
-// is stored per tap (TapHalf) and d/2 is computed once per hypothesis. The
+// is stored per tap and d/2 is computed once per hypothesis. The
 // coordinate is monotone in g, so the bounding box of the taps' g decides for
 // every tap at once whether all samples fall strictly inside [0, w-1) x [0, h-1);
 // inside, the reference's bounds checks and edge clamps cannot trigger and the
 // bilinear fetch reads the four neighbours from a quad plane with one 16-byte
-// load.
+// load (zncc_inside). Where grid_offset (common.cuh) also finds an f32 offset for both
+// coordinates, one f32 addition gives each (zncc_grid): most inside hypotheses of a plane
+// larger than a thumbnail.
 
 // Quad plane: the quad of (x, y) is (L[y][x], L[y][x1], L[y1][x], L[y1][x1]) with
 // x1 = min(x + 1, w - 1) and y1 = min(y + 1, h - 1), pair-interleaved: the quads of rows
@@ -447,59 +478,82 @@ __device__ __forceinline__ bool zncc_score(const PlaneRef &target, const TapT *g
 // taps of neighbouring labels spread along the epipolar line in any direction; against
 // row-major quads (8 x 1 per line) a 4 x 2 block keeps more of a quarter-warp's gathers
 // in one line.
-__host__ __device__ inline int quad_pair_stride(int width) { return 2 * ((width + 3) / 4 * 4); }
+__host__ __device__ inline int quad_stride(int width) { return 2 * ((width + 3) / 4 * 4); }
+inline size_t quad_count(int width, int height) { return (size_t)quad_stride(width) * ((height + 1) / 2); }
 
 __device__ __forceinline__ size_t quad_index(int x, int y, int stride) {
     return (size_t)(y >> 1) * stride + 2 * x + (y & 1);
 }
 
-__global__ void quad_plane_kernel(const float *__restrict__ plane, int width, int height, int stride,
-                                  float4 *quads) {
-    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)width * height) return;
-    int x = (int)(i % width), y = (int)(i / width);
-    long right = x + 1 < width ? 1 : 0, down = y + 1 < height ? width : 0;
-    quads[quad_index(x, y, stride)] = make_float4(plane[i], plane[i + right], plane[i + down], plane[i + down + right]);
-}
-
-struct TargetRef {
-    PlaneRef plane;
-    const float4 *quads;  // quad plane
+// Every target's planes for the correlations, in one launch: the quad plane, and for load_region
+// the plane and its transpose with rows padded to a multiple of 4 floats. A CTA of 32 x 8
+// threads makes a 32 x 32 tile of target blockIdx.y from one read of it and its right and lower
+// neighbours. HBM-bound: 4 B read, 24 B written per pixel.
+struct PlanesParams {
+    const DevView *views;
+    int targets[MAX_VIEWS];
 };
 
-// True when every tap at displacement (hdx, hdy) = (ddx/2, ddy/2) samples
-// strictly inside the plane.
-__device__ __forceinline__ bool taps_inside(const TapBox &box, double hdx, double hdy, int width, int height) {
-    float x0 = (float)((box.xmin + hdx) - 0.25), x1 = (float)((box.xmax + hdx) - 0.25);
-    float y0 = (float)((box.ymin + hdy) - 0.25), y1 = (float)((box.ymax + hdy) - 0.25);
-    // width, height < 2^22 (checked on the host), so inside also means < 2^22
-    return x0 >= 0.0f && y0 >= 0.0f && x1 < (float)(width - 1) && y1 < (float)(height - 1);
+__global__ void __launch_bounds__(256) sample_planes_kernel(PlanesParams p) {
+    __shared__ float tile[33][34];
+    const DevView &v = p.views[p.targets[blockIdx.y]];
+    const int width = v.luma.width, height = v.luma.height;
+    const int tiles_x = (width + 31) / 32, ty = blockIdx.x / tiles_x;
+    const int x0 = (blockIdx.x - ty * tiles_x) * 32, y0 = ty * 32, lane = threadIdx.x;
+    if (y0 >= height) return;
+    for (int i = threadIdx.y * 32 + lane; i < 33 * 33; i += 256) {
+        const int r = i / 33, c = i - r * 33;
+        tile[r][c] = __ldg(v.luma.data + (size_t)min(y0 + r, height - 1) * width + min(x0 + c, width - 1));
+    }
+    __syncthreads();
+    float4 *quads = const_cast<float4 *>(v.quads);
+    float *rows = const_cast<float *>(v.rows_plane.data), *columns = const_cast<float *>(v.columns_plane.data);
+    for (int r = threadIdx.y; r < 32; r += 8) {
+        int x = x0 + lane, y = y0 + r;
+        if (x < width && y < height) {
+            rows[(size_t)y * v.rows_plane.pitch + x] = tile[r][lane];
+            quads[quad_index(x, y, v.quad_stride)] =
+                make_float4(tile[r][lane], tile[r][lane + 1], tile[r + 1][lane], tile[r + 1][lane + 1]);
+        }
+        x = x0 + r;
+        y = y0 + lane;
+        if (x < width && y < height) columns[(size_t)x * v.columns_plane.pitch + y] = tile[lane][r];
+    }
 }
 
-// warped_patch_zncc's hypothesis-dependent part for taps known to be inside
-// (see taps_inside). gh holds g/2 per tap.
-template <typename TapT>
-__device__ __forceinline__ float zncc_inside(const float4 *__restrict__ quads, int stride, const TapT *gh,
-                                             const float2 *wt, const RefPatch &patch, int taps,
-                                             double hdx, double hdy, bool &ok) {
-    float st = 0.0f, stt = 0.0f, srt = 0.0f;
-#pragma unroll 9
-    for (int t = 0; t < taps; ++t) {
-        const double2 g = tap_half(gh[t]);
-        float x = (float)((g.x + hdx) - 0.25);
-        float y = (float)((g.y + hdy) - 0.25);
-        int ix, iy;
-        float tx = floor_frac_small(x, ix), ty = floor_frac_small(y, iy);
-        const float4 q = __ldg(quads + quad_index(ix, iy, stride));
-        float top = q.x * (1.0f - tx) + q.y * tx;
-        float bottom = q.z * (1.0f - tx) + q.w * tx;
-        float tv = top * (1.0f - ty) + bottom * ty;
-        const float2 weights = wt[t];
-        float wv = weights.x * tv;
-        st += wv;
-        stt += wv * tv;
-        srt += weights.y * tv;
-    }
+// The smallest and largest sample coordinates of a box displaced by (hdx, hdy) = (ddx/2, ddy/2).
+struct TapRange {
+    float x0, x1, y0, y1;
+};
+__device__ __forceinline__ TapRange tap_range(const TapBox &box, double hdx, double hdy) {
+    return {(float)(((double)box.xmin + hdx) - 0.25), (float)(((double)box.xmax + hdx) - 0.25),
+            (float)(((double)box.ymin + hdy) - 0.25), (float)(((double)box.ymax + hdy) - 0.25)};
+}
+
+// True when every tap samples strictly inside the plane.
+__device__ __forceinline__ bool taps_inside(const TapRange &r, int width, int height) {
+    // width, height < 2^22 (checked on the host), so inside also means < 2^22
+    return r.x0 >= 0.0f && r.y0 >= 0.0f && r.x1 < (float)(width - 1) && r.y1 < (float)(height - 1);
+}
+
+// True when every tap samples strictly inside the plane and one f32 addition of `offset`
+// per coordinate gives the reference's sample positions; `r` is then their range.
+__device__ __forceinline__ bool taps_on_grid(const TapBox &box, double ddx, double ddy, int width, int height,
+                                             float2 &offset, TapRange &r) {
+    if (max(width, height) > GRID_OFFSET_MAX_SIDE || !grid_offset(ddx * 0.5, box.xmin, offset.x) ||
+        !grid_offset(ddy * 0.5, box.ymin, offset.y))
+        return false;
+    r = {box.xmin + offset.x, box.xmax + offset.x, box.ymin + offset.y, box.ymax + offset.y};
+    return taps_inside(r, width, height);
+}
+__device__ __forceinline__ bool taps_on_grid(const TapBox &box, double ddx, double ddy, int width, int height,
+                                             float2 &offset) {
+    TapRange r;
+    return taps_on_grid(box, ddx, ddy, width, height, offset, r);
+}
+
+// The correlation from the three target sums (depth.rs:1815-1822).
+__device__ __forceinline__ float zncc_finish(const RefPatch &patch, float st, float stt, float srt, bool &ok) {
     float covariance = srt - patch.sum_r * st / patch.count;
     float target_energy = stt - st * st / patch.count;
     float denominator = sqrtf(fmaxf(patch.ref_energy, 0.0f) * fmaxf(target_energy, 0.0f));
@@ -507,18 +561,186 @@ __device__ __forceinline__ float zncc_inside(const float4 *__restrict__ quads, i
     return clampf_r(covariance / denominator, -1.0f, 1.0f);
 }
 
-// Either path, bit-identical to warped_patch_zncc: fast when the box is inside,
-// exact per-tap checks otherwise. gh: g/2 per tap.
-template <typename TapT>
-__device__ __forceinline__ bool zncc_any(const TargetRef &target, const TapT *gh, const TapBox &box, const float2 *wt, const RefPatch &patch,
-                                         int taps, double ddx, double ddy, float &score) {
-    double hdx = ddx * 0.5, hdy = ddy * 0.5;
-    if (taps_inside(box, hdx, hdy, target.plane.width, target.plane.height)) {
+// The bilinear sample of a quad and its three sums.
+__device__ __forceinline__ void add_sample(const float4 &q, float2 frac, float2 rest, float2 weights, float &st,
+                                           float &stt, float &srt) {
+    float top = q.x * rest.x + q.y * frac.x;
+    float bottom = q.z * rest.x + q.w * frac.x;
+    float tv = top * rest.y + bottom * frac.y;
+    float wv = weights.x * tv;
+    st += wv;
+    stt += wv * tv;
+    srt += weights.y * tv;
+}
+
+// warped_patch_zncc's hypothesis-dependent part for taps known to be inside
+// (see taps_inside).
+template <int UNROLL, typename TapT>
+__device__ __forceinline__ float zncc_inside(const float4 *__restrict__ quads, int stride, TapT gh,
+                                             const float2 *wt, const RefPatch &patch, int taps,
+                                             double hdx, double hdy, bool &ok) {
+    float st = 0.0f, stt = 0.0f, srt = 0.0f;
+#pragma unroll UNROLL
+    for (int t = 0; t < taps; ++t) {
+        const auto tap = load_tap(gh, wt, t);
+        const float x = (float)(((double)tap.half.x + hdx) - 0.25);
+        const float y = (float)(((double)tap.half.y + hdy) - 0.25);
+        const float mx = __fadd_rd(x, 8388608.0f), my = __fadd_rd(y, 8388608.0f);  // 2^23 + floor
+        const float tx = x - (mx - 8388608.0f), ty = y - (my - 8388608.0f);
+        const float4 q = __ldg(quads + quad_index((int)(f2u(mx) - 0x4B000000u), (int)(f2u(my) - 0x4B000000u), stride));
+        add_sample(q, make_float2(tx, ty), make_float2(1.0f - tx, 1.0f - ty), tap.weights, st, stt, srt);
+    }
+    return zncc_finish(patch, st, stt, srt, ok);
+}
+
+// The same for taps that taps_on_grid accepted, with its offset. The two coordinates go
+// through packed f32 instructions (two IEEE operations in one): the addition; the floor, by
+// adding 2^23 rounded down (0 <= x < 2^22, so the sum is 2^23 + floor(x) and its low bits
+// hold the index); the fraction x - floor(x), exact; and 1 - fraction, rounded once.
+template <int UNROLL, typename TapT>
+__device__ __forceinline__ float zncc_grid(const float4 *__restrict__ quads, int stride, TapT gh,
+                                           const float2 *wt, const RefPatch &patch, int taps, float2 offset,
+                                           bool &ok) {
+    const f32x2 e = pack2(offset.x, offset.y), magic = pack2(8388608.0f, 8388608.0f);
+    const f32x2 minus_magic = pack2(-8388608.0f, -8388608.0f), one = pack2(1.0f, 1.0f);
+    const f32x2 minus_one = pack2(-1.0f, -1.0f);
+    float st = 0.0f, stt = 0.0f, srt = 0.0f;
+#pragma unroll UNROLL
+    for (int t = 0; t < taps; ++t) {
+        const auto tap = load_tap(gh, wt, t);
+        const f32x2 x = add2(pack2(tap.half.x, tap.half.y), e);
+        const f32x2 m = add2_down(x, magic);
+        const f32x2 frac = fma2(add2(m, minus_magic), minus_one, x), rest = fma2(frac, minus_one, one);
+        const float2 mf = unpack2(m);
+        const int ix = (int)(f2u(mf.x) - 0x4B000000u), iy = (int)(f2u(mf.y) - 0x4B000000u);
+        const float4 q = __ldg(quads + quad_index(ix, iy, stride));
+        add_sample(q, unpack2(frac), unpack2(rest), tap.weights, st, stt, srt);
+    }
+    return zncc_finish(patch, st, stt, srt, ok);
+}
+
+// ---- samples from a region in shared memory ------------------------------------------
+// A warp's lanes score neighbouring hypotheses: at one tap their samples lie along the
+// target's epipolar line, half a pixel to two pixels apart. Gathered from the quad plane
+// those are 20 to 30 128-byte lines an instruction, about 13 passes through the L1's data
+// stage. From a copy of the rectangle around the whole segment, one float per pixel, the
+// four neighbours of a sample are four 4-byte shared loads. Lanes in different banks cost
+// nothing there, so the copy is laid out with its rows along the coordinate axis nearer to
+// the epipolar line (the target's plane or its transpose) and a row pitch of a multiple of
+// 32 words: the bank is the position along that axis, in which neighbouring lanes differ.
+constexpr int REGION_PITCH = 96;  // a reach of 64 samples (128 px displacement), a patch, a tile and alignment
+
+struct Region {
+    int column, row, columns, rows;  // of the stored plane (transposed or not); column a multiple of 4
+};
+
+// The rectangle of a range of sample floors (lowest x, lowest y, -highest x, -highest y) and
+// each one's right and lower neighbour. False where it does not fit the buffer.
+__device__ __forceinline__ bool region_of(const int *range, bool transposed, int rows, Region &r) {
+    const int c0 = range[transposed ? 1 : 0], r0 = range[transposed ? 0 : 1];
+    const int c1 = -range[transposed ? 3 : 2], r1 = -range[transposed ? 2 : 3];
+    r.column = c0 & ~3;
+    r.row = r0;
+    r.columns = c1 + 2 - r.column;
+    r.rows = r1 + 2 - r0;
+    return r.columns <= REGION_PITCH && r.rows <= rows;
+}
+
+// Copies a region with 16-byte asynchronous copies (copy_async_wait, then a barrier). The
+// plane's rows are padded to its pitch, a multiple of 4, so a copy that starts inside a row
+// ends inside it.
+__device__ __forceinline__ void load_region(const Region &r, const PaddedPlane &plane, float *region, int tid,
+                                            int threads) {
+    const int quarters = (r.columns + 3) >> 2;
+    const int groups = threads / 24;  // of 24 threads: a whole row
+    const int row0 = tid / 24, at = tid - row0 * 24;
+    if (row0 >= groups || at >= quarters) return;
+    const float *src = plane.data + (size_t)(r.row + row0) * plane.pitch + r.column + 4 * at;
+    uint32_t dst = (uint32_t)__cvta_generic_to_shared(region + row0 * REGION_PITCH + 4 * at);
+    for (int row = row0; row < r.rows; row += groups) {
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        src += (size_t)groups * plane.pitch;
+        dst += groups * REGION_PITCH * sizeof(float);
+    }
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// The samples' coordinates of a pair of taps: one f32 addition each for a hypothesis on the grid
+// (place: its offset), else in f64 (place: half its displacement; see taps_inside).
+__device__ __forceinline__ void pair_position(const float4 &half, const float2 &place, f32x2 &x, f32x2 &y) {
+    x = add2(pack2(half.x, half.y), pack2(place.x, place.x));
+    y = add2(pack2(half.z, half.w), pack2(place.y, place.y));
+}
+__device__ __forceinline__ void pair_position(const float4 &half, const double2 &place, f32x2 &x, f32x2 &y) {
+    x = pack2((float)(((double)half.x + place.x) - 0.25), (float)(((double)half.y + place.x) - 0.25));
+    y = pack2((float)(((double)half.z + place.y) - 0.25), (float)(((double)half.w + place.y) - 0.25));
+}
+
+// zncc_grid or zncc_inside with the samples in a region, two taps at a time in packed arithmetic
+// (the sums take them in tap order). opaque_one: see add2_products.
+template <bool TRANSPOSED, typename Place>
+__device__ __forceinline__ float zncc_region(const float *region, const Region &r, const PairedTaps &tap,
+                                             const RefPatch &patch, int taps, const Place &place, float opaque_one,
+                                             bool &ok) {
+    constexpr unsigned SX = TRANSPOSED ? REGION_PITCH : 1, SY = TRANSPOSED ? 1 : REGION_PITCH;
+    const f32x2 magic = pack2(8388608.0f, 8388608.0f), minus_magic = pack2(-8388608.0f, -8388608.0f);
+    const f32x2 one = pack2(opaque_one, opaque_one), minus_one = pack2(-1.0f, -1.0f);
+    // word of a sample: bits(2^23 + x) SX + bits(2^23 + y) SY + c
+    const unsigned c = 0u - (0x4B000000u + (unsigned)(TRANSPOSED ? r.row : r.column)) * SX -
+                       (0x4B000000u + (unsigned)(TRANSPOSED ? r.column : r.row)) * SY;
+    float st = 0.0f, stt = 0.0f, srt = 0.0f;
+#pragma unroll 1
+    for (int t = 0; t < taps >> 1; ++t) {
+        const float4 b = tap.weight[t];
+        f32x2 x, y;
+        pair_position(tap.half[t], place, x, y);
+        const f32x2 mx = add2_down(x, magic), my = add2_down(y, magic);
+        const f32x2 fx = fma2(add2(mx, minus_magic), minus_one, x), fy = fma2(add2(my, minus_magic), minus_one, y);
+        const f32x2 ux = fma2(fx, minus_one, one), uy = fma2(fy, minus_one, one);
+        const float2 mxf = unpack2(mx), myf = unpack2(my);
+        const float *q0 = region + (f2u(mxf.x) * SX + f2u(myf.x) * SY + c);
+        const float *q1 = region + (f2u(mxf.y) * SX + f2u(myf.y) * SY + c);
+        const f32x2 top = add2_products(mul2(pack2(q0[0], q1[0]), ux), mul2(pack2(q0[SX], q1[SX]), fx), one);
+        const f32x2 bottom =
+            add2_products(mul2(pack2(q0[SY], q1[SY]), ux), mul2(pack2(q0[SX + SY], q1[SX + SY]), fx), one);
+        const f32x2 tv = add2_products(mul2(top, uy), mul2(bottom, fy), one);
+        const f32x2 wv = mul2(pack2(b.x, b.y), tv);
+        const float2 s0 = unpack2(wv), s1 = unpack2(mul2(wv, tv)), s2 = unpack2(mul2(pack2(b.z, b.w), tv));
+        st += s0.x;
+        stt += s1.x;
+        srt += s2.x;
+        st += s0.y;
+        stt += s1.y;
+        srt += s2.y;
+    }
+    {
+        const float4 b = tap.weight[taps >> 1];
+        f32x2 last_x, last_y;
+        pair_position(tap.half[taps >> 1], place, last_x, last_y);
+        const float x = unpack2(last_x).x, y = unpack2(last_y).x;
+        const float mx = __fadd_rd(x, 8388608.0f), my = __fadd_rd(y, 8388608.0f);
+        const float tx = x - (mx - 8388608.0f), ty = y - (my - 8388608.0f);
+        const float *q = region + (f2u(mx) * SX + f2u(my) * SY + c);
+        add_sample(make_float4(q[0], q[SX], q[SY], q[SX + SY]), make_float2(tx, ty), make_float2(1.0f - tx, 1.0f - ty),
+                   make_float2(b.x, b.z), st, stt, srt);
+    }
+    return zncc_finish(patch, st, stt, srt, ok);
+}
+
+// Either path in f64, bit-identical to warped_patch_zncc: the fast loop when the box is inside,
+// exact per-tap checks otherwise.
+template <int UNROLL, typename TapT>
+__device__ __forceinline__ bool zncc_any(const DevView &target, TapT gh, const TapBox &box,
+                                              const float2 *wt, const RefPatch &patch, int taps, double ddx,
+                                              double ddy, float &score) {
+    const PlaneRef &plane = target.luma;
+    const double hdx = ddx * 0.5, hdy = ddy * 0.5;
+    if (taps_inside(tap_range(box, hdx, hdy), plane.width, plane.height)) {
         bool ok;
-        score = zncc_inside(target.quads, quad_pair_stride(target.plane.width), gh, wt, patch, taps, hdx, hdy, ok);
+        score = zncc_inside<UNROLL>(target.quads, target.quad_stride, gh, wt, patch, taps, hdx, hdy, ok);
         return ok;
     }
-    return zncc_score(target.plane, gh, wt, patch, taps, ddx, ddy, score);
+    return zncc_score(plane, gh, wt, patch, taps, ddx, ddy, score);
 }
 
 // aggregate (depth.rs:1761-1770) over up to MAX_VIEWS scores (NaN = None).
