@@ -355,11 +355,30 @@ __device__ inline bool decisions_agree(int kind, uint8_t ck, float2 cg, float2 c
     return kind == 1 && ck == CHIARO_NW_OCCLUDED && nk == CHIARO_NW_OCCLUDED;
 }
 
-// enforce_warp_consensus: reads `src`, writes `dst` (a copy on entry).
-__global__ void warp_consensus_kernel(Decisions src, Decisions dst, int columns, int rows) {
+// The passes after the decisions, every target (blockIdx.y) in one launch. A node that consensus
+// or a boundary overrules keeps its mappings and only changes its kind (its point becomes its
+// global mapping, which every reader takes for those kinds), so a pass writes one byte per node
+// instead of a copy of all five arrays.
+struct WarpPasses {
+    Decisions decisions[MAX_VIEWS];
+    uint8_t *agreed;  // [target][node] kinds after enforce_warp_consensus
+    uint8_t *kinds;   // [target][node] kinds after suppress_warp_boundaries, or nullptr
+    const float *guidance;
+    float2 *points[MAX_VIEWS];  // output warps, or nullptr
+    float *confidence[MAX_VIEWS];
+    unsigned long long *counts[MAX_VIEWS];  // refined, occluded, boundary
+    int columns, rows;
+};
+
+// enforce_warp_consensus (depth.rs:582-618)
+__global__ void warp_consensus_kernel(WarpPasses p) {
+    const int columns = p.columns, rows = p.rows;
     int index = blockIdx.x * blockDim.x + threadIdx.x;
     if (index >= columns * rows) return;
+    const Decisions &src = p.decisions[blockIdx.y];
+    uint8_t *const agreed = p.agreed + (size_t)blockIdx.y * columns * rows;
     uint8_t k = src.kind[index];
+    agreed[index] = k;
     int kind, minimum;
     if (k == CHIARO_NW_REFINED) {
         kind = 0;
@@ -381,17 +400,11 @@ __global__ void warp_consensus_kernel(Decisions src, Decisions dst, int columns,
             int ni = y * columns + x;
             neighbours += decisions_agree(kind, k, cg, cp, src.kind[ni], src.global[ni], src.point[ni]) ? 1 : 0;
         }
-    if (neighbours < minimum) {
-        dst.kind[index] = CHIARO_NW_GLOBAL;
-        dst.point[index] = cg;
-        dst.confidence[index] = 0.0f;
-        dst.measured[index] = 0;
-    }
+    if (neighbours < minimum) agreed[index] = CHIARO_NW_GLOBAL;
 }
 
-// warp_mapping (depth.rs:674-680)
-__device__ inline bool decision_mapping(const Decisions &d, int i, float2 &g, float2 &pt) {
-    uint8_t k = d.kind[i];
+// warp_mapping (depth.rs:674-680) of a node of kind k
+__device__ inline bool decision_mapping(const Decisions &d, uint8_t k, int i, float2 &g, float2 &pt) {
     if (k == CHIARO_NW_GLOBAL) {
         g = d.global[i];
         pt = g;
@@ -406,9 +419,9 @@ __device__ inline bool decision_mapping(const Decisions &d, int i, float2 &g, fl
 }
 
 // Does the 4-connected pair (a, b), a west/north of b, form a warp boundary?
-__device__ inline bool boundary_pair(const Decisions &d, const float *guidance, int a, int b) {
+__device__ inline bool boundary_pair(const Decisions &d, const uint8_t *kinds, const float *guidance, int a, int b) {
     float2 ga, pa, gb, pb;
-    if (!decision_mapping(d, a, ga, pa) || !decision_mapping(d, b, gb, pb)) return false;
+    if (!decision_mapping(d, kinds[a], a, ga, pa) || !decision_mapping(d, kinds[b], b, gb, pb)) return false;
     float dax = pa.x - ga.x, day = pa.y - ga.y;
     float dbx = pb.x - gb.x, dby = pb.y - gb.y;
     float ex = dax - dbx, ey = day - dby;
@@ -417,52 +430,47 @@ __device__ inline bool boundary_pair(const Decisions &d, const float *guidance, 
     return mapping_edge && image_edge;
 }
 
-// suppress_warp_boundaries: reads `src`, writes `dst` (a copy on entry).
-__global__ void warp_boundary_kernel(Decisions src, Decisions dst, const float *__restrict__ guidance, int columns,
-                                     int rows) {
-    int index = blockIdx.x * blockDim.x + threadIdx.x;
-    if (index >= columns * rows) return;
-    float2 g, pt;
-    if (!decision_mapping(src, index, g, pt)) return;
-    int column = index % columns, row = index / columns;
-    bool boundary = (column + 1 < columns && boundary_pair(src, guidance, index, index + 1)) ||
-                    (row + 1 < rows && boundary_pair(src, guidance, index, index + columns)) ||
-                    (column > 0 && boundary_pair(src, guidance, index - 1, index)) ||
-                    (row > 0 && boundary_pair(src, guidance, index - columns, index));
-    if (boundary) {
-        dst.kind[index] = CHIARO_NW_BOUNDARY;
-        dst.point[index] = g;
-        dst.confidence[index] = 0.0f;
-    }
-}
-
-// Output warp and decision counts (depth.rs:490-532). counts: refined,
-// occluded, boundary.
-__global__ void warp_output_kernel(Decisions d, float2 *points, float *confidence,
-                                   unsigned long long *counts, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+// suppress_warp_boundaries (depth.rs:620-672), the output warp and decision counts
+// (depth.rs:490-532).
+__global__ void warp_output_kernel(WarpPasses p) {
+    const int columns = p.columns, rows = p.rows, n = columns * rows, v = blockIdx.y;
+    const int index = blockIdx.x * blockDim.x + threadIdx.x;
     int refined = 0, occluded = 0, boundary = 0;
-    if (i < n) {
-        uint8_t k = d.kind[i];
+    if (index < n) {
+        const Decisions &d = p.decisions[v];
+        const uint8_t *const kinds = p.agreed + (size_t)v * n;
+        uint8_t k = kinds[index];
+        if (k == CHIARO_NW_GLOBAL || k == CHIARO_NW_REFINED) {
+            const int column = index % columns, row = index / columns;
+            if ((column + 1 < columns && boundary_pair(d, kinds, p.guidance, index, index + 1)) ||
+                (row + 1 < rows && boundary_pair(d, kinds, p.guidance, index, index + columns)) ||
+                (column > 0 && boundary_pair(d, kinds, p.guidance, index - 1, index)) ||
+                (row > 0 && boundary_pair(d, kinds, p.guidance, index - columns, index)))
+                k = CHIARO_NW_BOUNDARY;
+        }
+        if (p.kinds) p.kinds[(size_t)v * n + index] = k;
         float2 pt;
         float c;
         switch (k) {
             case CHIARO_NW_UNDEFINED: pt = make_float2(NAN, NAN); c = 0.0f; break;
-            case CHIARO_NW_GLOBAL: pt = d.global[i]; c = 1.0f; break;
-            case CHIARO_NW_REFINED: pt = d.point[i]; c = d.confidence[i]; refined = 1; break;
-            case CHIARO_NW_OCCLUDED: pt = d.global[i]; c = 0.0f; occluded = 1; break;
-            default: pt = d.global[i]; c = 0.0f; boundary = 1; break;
+            case CHIARO_NW_GLOBAL: pt = d.global[index]; c = 1.0f; break;
+            case CHIARO_NW_REFINED: pt = d.point[index]; c = d.confidence[index]; refined = 1; break;
+            case CHIARO_NW_OCCLUDED: pt = d.global[index]; c = 0.0f; occluded = 1; break;
+            default: pt = d.global[index]; c = 0.0f; boundary = 1; break;
         }
-        points[i] = pt;
-        confidence[i] = c;
+        if (p.points[v]) {
+            p.points[v][index] = pt;
+            p.confidence[v][index] = c;
+        }
     }
+    if (!p.counts[v]) return;
     unsigned full = 0xffffffffu;
     int rc = __popc(__ballot_sync(full, refined)), oc = __popc(__ballot_sync(full, occluded)),
         bc = __popc(__ballot_sync(full, boundary));
     if ((threadIdx.x & 31) == 0) {
-        if (rc) atomicAdd(counts + 0, (unsigned long long)rc);
-        if (oc) atomicAdd(counts + 1, (unsigned long long)oc);
-        if (bc) atomicAdd(counts + 2, (unsigned long long)bc);
+        if (rc) atomicAdd(p.counts[v] + 0, (unsigned long long)rc);
+        if (oc) atomicAdd(p.counts[v] + 1, (unsigned long long)oc);
+        if (bc) atomicAdd(p.counts[v] + 2, (unsigned long long)bc);
     }
 }
 

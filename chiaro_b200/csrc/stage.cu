@@ -7,8 +7,6 @@
 // stage is a kernel; the host only validates, uploads, launches and reads
 // the results back. There is no CPU fallback: a CUDA failure is reported as
 // CHIARO_ERR_CUDA.
-#include <cub/cub.cuh>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -24,6 +22,7 @@
 #include "filters.cuh"
 #include "luminance.cuh"
 #include "select.cuh"
+#include "stats.cuh"
 #include "sgm.cuh"
 #include "sgm_u16.cuh"
 #include "sgm_batch.cuh"
@@ -1272,7 +1271,6 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         CK(cudaEventRecord(ctx->events[2], s));
         CK(cudaEventRecord(ctx->events[3], s));
         float *scores = dbuf<float>(ctx, "coarse.scores", N * D), *costs = dbuf<float>(ctx, "coarse.costs", N * D);
-        CK(cudaMemsetAsync(tested, 0, N, s));
         coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, nullptr, N, scores, costs, guidance, tested);
         CK(cudaEventRecord(ctx->events[4], s));
         float *aggregate = dbuf<float>(ctx, "coarse.aggregate", N * D);
@@ -1292,7 +1290,6 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         upload(ctx, d_list, list.data(), PREPASS_SLOTS);
         float *pre_scores = dbuf<float>(ctx, "coarse.prepass_scores", N * PREPASS_SLOTS);
         float *pre_costs = dbuf<float>(ctx, "coarse.prepass_costs", N * PREPASS_SLOTS);
-        CK(cudaMemsetAsync(tested, 0, N, s));
         coarse_cost(ctx, g, reference, o, PREPASS_SLOTS, d_list, nullptr, nullptr, N, pre_scores, pre_costs, guidance,
                     tested);
         CK(cudaEventRecord(ctx->events[2], s));
@@ -1325,7 +1322,6 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         float *band_costs = dbuf<float>(ctx, "coarse.band_costs", N * (1 + band));
         uint8_t *band_tested = dbuf<uint8_t>(ctx, "coarse.band_tested", N);
         float *band_guidance = dbuf<float>(ctx, "coarse.band_guidance", N);
-        CK(cudaMemsetAsync(band_tested, 0, N, s));
         coarse_cost(ctx, g, reference, o, 1 + band, nullptr, &grid, nullptr, N, band_scores, band_costs,
                     band_guidance, band_tested);
         CK(cudaEventRecord(ctx->events[4], s));
@@ -1446,59 +1442,6 @@ struct HostTransfers {
     float *warp_confidence[MAX_VIEWS] = {};
 };
 
-struct Results {  // read back once at the end
-    int status;  // UNION_GAVE_UP when a component join ran out of retries
-    unsigned long long tested, measured, regularized;
-    unsigned long long target_counts[MAX_VIEWS][3];
-    double median_depth;
-    float median_improvement;
-    int has_median_depth, has_median_improvement;
-};
-
-__global__ void field_stats_kernel(const uint8_t *__restrict__ tested, Field f, int n, Results *res, double *depth_keys,
-                                   float *improvement_keys) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int t = 0, m = 0, r = 0;
-    if (i < n) {
-        t = tested[i];
-        bool has = f.has[i];
-        m = has && !f.regularized[i];
-        r = has && f.regularized[i];
-        depth_keys[i] = has ? f.depth[i] : INFINITY;
-        improvement_keys[i] = m ? f.improvement[i] : INFINITY;
-    }
-    unsigned full = 0xffffffffu;
-    int ct = __popc(__ballot_sync(full, t)), cm = __popc(__ballot_sync(full, m)), cr = __popc(__ballot_sync(full, r));
-    if ((threadIdx.x & 31) == 0) {
-        if (ct) atomicAdd(&res->tested, (unsigned long long)ct);
-        if (cm) atomicAdd(&res->measured, (unsigned long long)cm);
-        if (cr) atomicAdd(&res->regularized, (unsigned long long)cr);
-    }
-}
-
-__global__ void medians_kernel(const double *sorted_depth, const float *sorted_improvement, Results *res) {
-    unsigned long long nd = res->measured + res->regularized, ni = res->measured;
-    res->has_median_depth = nd > 0;
-    res->median_depth = nd > 0 ? sorted_depth[nd / 2] : 0.0;
-    res->has_median_improvement = ni > 0;
-    res->median_improvement = ni > 0 ? sorted_improvement[ni / 2] : 0.0f;
-}
-
-__global__ void depth_map_kernel(Field f, const uint8_t *__restrict__ tested, double *depth, float *confidence,
-                                 uint8_t *provenance, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (f.has[i]) {
-        depth[i] = f.depth[i];
-        confidence[i] = f.confidence[i];
-        provenance[i] = f.regularized[i] ? CHIARO_REGULARIZED : CHIARO_MEASURED;
-    } else {
-        depth[i] = NAN;
-        confidence[i] = tested[i] ? 1.0f : 0.0f;
-        provenance[i] = tested[i] ? CHIARO_GLOBAL : CHIARO_UNSUPPORTED;
-    }
-}
-
 Field field_bufs(chiaro_depth_ctx *ctx, const std::string &name, size_t n) {
     Field f;
     f.has = dbuf<uint8_t>(ctx, name + ".has", n);
@@ -1525,14 +1468,6 @@ Decisions decision_bufs(chiaro_depth_ctx *ctx, const std::string &name, size_t n
     d.confidence = dbuf<float>(ctx, name + ".confidence", n);
     d.measured = dbuf<uint8_t>(ctx, name + ".measured", n);
     return d;
-}
-
-void copy_decisions(chiaro_depth_ctx *ctx, const Decisions &dst, const Decisions &src, size_t n) {
-    CK(cudaMemcpyAsync(dst.kind, src.kind, n, cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dst.global, src.global, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dst.point, src.point, n * 8, cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dst.confidence, src.confidence, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(dst.measured, src.measured, n, cudaMemcpyDeviceToDevice, ctx->stream));
 }
 
 void download_field(chiaro_depth_ctx *ctx, const Field &f, size_t n, uint8_t *has, double *depth, float *confidence,
@@ -1657,18 +1592,21 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     std::vector<double> spatial25(25);
     for (int dy = -2; dy <= 2; ++dy)
         for (int dx = -2; dx <= 2; ++dx) spatial25[(dy + 2) * 5 + dx + 2] = std::exp((double)(-(dx * dx + dy * dy)) / 6.0);
-    double *d_labels = dbuf<double>(ctx, "labels", D);
-    double *d_unseeded = dbuf<double>(ctx, "unseeded", 32);
-    float *d_sp = dbuf<float>(ctx, "spatial", sp.size());
-    float *d_sp_direct = dbuf<float>(ctx, "spatial_direct", sp_direct.size());
-    float *d_sp_wide = dbuf<float>(ctx, "spatial_wide", sp_wide.size());
-    double *d_sp25 = dbuf<double>(ctx, "spatial25", 25);
-    upload(ctx, d_labels, labels.data(), D);
-    upload(ctx, d_unseeded, unseeded.data(), 32);
-    upload(ctx, d_sp, sp.data(), sp.size());
-    upload(ctx, d_sp_direct, sp_direct.data(), sp_direct.size());
-    upload(ctx, d_sp_wide, sp_wide.data(), sp_wide.size());
-    upload(ctx, d_sp25, spatial25.data(), 25);
+    // one upload: the f64 tables, then the f32 ones
+    const size_t doubles = D + 32 + 25, floats = sp.size() + sp_direct.size() + sp_wide.size();
+    std::vector<double> tables(doubles + (floats + 1) / 2);
+    std::copy(labels.begin(), labels.end(), tables.begin());
+    std::copy(unseeded.begin(), unseeded.end(), tables.begin() + D);
+    std::copy(spatial25.begin(), spatial25.end(), tables.begin() + D + 32);
+    float *h_floats = reinterpret_cast<float *>(tables.data() + doubles);
+    std::copy(sp.begin(), sp.end(), h_floats);
+    std::copy(sp_direct.begin(), sp_direct.end(), h_floats + sp.size());
+    std::copy(sp_wide.begin(), sp_wide.end(), h_floats + sp.size() + sp_direct.size());
+    double *d_labels = dbuf<double>(ctx, "tables", tables.size());
+    double *d_unseeded = d_labels + D, *d_sp25 = d_unseeded + 32;
+    float *d_sp = reinterpret_cast<float *>(d_labels + doubles), *d_sp_direct = d_sp + sp.size();
+    float *d_sp_wide = d_sp_direct + sp_direct.size();
+    upload(ctx, d_labels, tables.data(), tables.size());
     // the quad planes' buffers and the views that point at them, before any launch
     for (int t : targets) sample_planes(ctx, t, h_views[t]);
     upload(ctx, d_views, h_views.data(), h_views.size());
@@ -1693,9 +1631,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         lattice.planes = dbuf<float2>(ctx, "tap_lattice", (size_t)(V + 1) * lattice.columns * lattice.rows);
     }
     // sample planes and geometry 1 each, tap lattice 1, patches 1, cost 1, SGM 2, select 1, completion, direct 2,
-    // filters 6, stats 2, decisions 1 + 3 per target, map 1
+    // filters 6, map and statistics 5, decisions 3
     ctx->launches = (V > 0 ? 2 : 0) + (lattice.planes ? 1 : 0) + 1 + 1 + 2 + 1 + (int)o.completion_iterations + 2 + 6 +
-                    2 + (V > 0 ? 1 + 3 * V : 0) + 1;
+                    SELECT_PASSES + (V > 0 ? 3 : 0);
     // the whole-stage graph (device-buffer calls only)
     ctx->stage_graph_state = 0;
     bool capturing = false;
@@ -1779,7 +1717,6 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     float *costs = dbuf<float>(ctx, "costs", N * D);
     float *guidance = dbuf<float>(ctx, "guidance", N);
     uint8_t *tested = dbuf<uint8_t>(ctx, "tested", N);
-    CK(cudaMemsetAsync(tested, 0, N, s));  // the cost kernel only sets tested nodes
     {
         CostParams p{};
         p.geometry = coarse_geometry;
@@ -1937,7 +1874,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
                                                                (int)g.rows, inverse_step * 2.5,
                                                                union_retries(ctx, M), &d_results->status);
     components_size_kernel<<<blocks_for(M, 256), 256, 0, s>>>(has_a, parent, csize, (int)M);
-    Field fin = field_bufs(ctx, "final", M);
+    Field fin = direct;  // what the filters leave as it is
+    fin.has = dbuf<uint8_t>(ctx, "final.has", M);
+    fin.depth = dbuf<double>(ctx, "final.depth", M);
     components_mark_kernel<<<blocks_for(M, 256), 256, 0, s>>>(has_a, parent, csize, fin.has, (int)M,
                                                               MINIMUM_DIRECT_COMPONENT_NODES);
     CK(cudaGetLastError());
@@ -1946,9 +1885,6 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
                                                                d_sp25, fin.depth, (int)g.columns, (int)g.rows,
                                                                inverse_step * 4.0);
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(fin.confidence, direct.confidence, M * 4, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(fin.improvement, direct.improvement, M * 4, cudaMemcpyDeviceToDevice, s));
-    CK(cudaMemcpyAsync(fin.regularized, direct.regularized, M, cudaMemcpyDeviceToDevice, s));
     // depth of removed nodes: NaN (None)
     if (debug && debug->fitted_depth) {
         std::vector<uint8_t> h(M);
@@ -1958,26 +1894,24 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         for (size_t i = 0; i < M; ++i)
             if (!h[i]) debug->fitted_depth[i] = NAN;
     }
-    // report statistics and medians
-    double *depth_keys = dbuf<double>(ctx, "depth_keys", M);
-    double *depth_sorted = dbuf<double>(ctx, "depth_sorted", M);
-    float *imp_keys = dbuf<float>(ctx, "imp_keys", M);
-    float *imp_sorted = dbuf<float>(ctx, "imp_sorted", M);
-    field_stats_kernel<<<blocks_for(M, 256), 256, 0, s>>>(ftested, fin, (int)M, d_results, depth_keys, imp_keys);
-    CK(cudaGetLastError());
+    // the depth map (it needs only the final field, so it is ready before the decisions),
+    // the report's counts and medians
     {
-        size_t t1 = 0, t2 = 0;
-        CK(cub::DeviceRadixSort::SortKeys(nullptr, t1, depth_keys, depth_sorted, (int)M, 0, 64, s));
-        CK(cub::DeviceRadixSort::SortKeys(nullptr, t2, imp_keys, imp_sorted, (int)M, 0, 32, s));
-        void *tmp = dbuf<unsigned char>(ctx, "cub_tmp", std::max(t1, t2));
-        CK(cub::DeviceRadixSort::SortKeys(tmp, t1, depth_keys, depth_sorted, (int)M, 0, 64, s));
-        CK(cub::DeviceRadixSort::SortKeys(tmp, t2, imp_keys, imp_sorted, (int)M, 0, 32, s));
+        StatsParams p{};
+        p.field = fin;
+        p.tested = ftested;
+        p.n = (int)M;
+        p.results = d_results;
+        p.state = dbuf<SelectState>(ctx, "select_state", 1);
+        p.depth = out.depth;
+        p.confidence = out.confidence;
+        p.provenance = out.provenance;
+        CK(cudaMemsetAsync(p.state, 0, sizeof(SelectState), s));
+        const unsigned blocks = (unsigned)std::min<size_t>(div_ceil(M, 256), (size_t)ctx->sm_count * 4);
+        field_stats_kernel<true><<<dim3(blocks, 2), 256, 0, s>>>(p);
+        for (p.pass = 1; p.pass < SELECT_PASSES; ++p.pass) field_stats_kernel<false><<<dim3(blocks, 2), 256, 0, s>>>(p);
+        CK(cudaGetLastError());
     }
-    medians_kernel<<<1, 1, 0, s>>>(depth_sorted, imp_sorted, d_results);
-    CK(cudaGetLastError());
-    // the depth map needs only the final field, so it is ready before the decisions
-    depth_map_kernel<<<blocks_for(M, 256), 256, 0, s>>>(fin, ftested, out.depth, out.confidence, out.provenance, (int)M);
-    CK(cudaGetLastError());
     if (host) CK(cudaEventRecord(ctx->map_ready, s));
     record_event(ctx->events[5], s, capturing);
     // ---- per-target decisions (depth.rs:420-547): all targets in one launch
@@ -2013,21 +1947,25 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         const int warps = warps_per_cta(decision_kernel, slot, DECISION_WARPS);
         decision_kernel<<<blocks_for(M, warps), 32 * warps, warps * slot, s>>>(p);
         CK(cudaGetLastError());
-        Decisions dec2 = decision_bufs(ctx, "dec_consensus", M), dec3 = decision_bufs(ctx, "dec_boundary", M);
+        WarpPasses w{};
+        w.agreed = dbuf<uint8_t>(ctx, "dec_agreed", V * M);
+        if (debug && debug->decision_kind) w.kinds = dbuf<uint8_t>(ctx, "dec_kinds", V * M);
+        w.guidance = fguidance;
+        w.columns = (int)g.columns;
+        w.rows = (int)g.rows;
         for (int v = 0; v < V; ++v) {
             const int t = targets[v];
-            const Decisions &dec = p.out[v];
-            copy_decisions(ctx, dec2, dec, M);
-            warp_consensus_kernel<<<blocks_for(M, 256), 256, 0, s>>>(dec, dec2, (int)g.columns, (int)g.rows);
-            copy_decisions(ctx, dec3, dec2, M);
-            warp_boundary_kernel<<<blocks_for(M, 256), 256, 0, s>>>(dec2, dec3, fguidance, (int)g.columns,
-                                                                    (int)g.rows);
-            warp_output_kernel<<<blocks_for(M, 256), 256, 0, s>>>(dec3, out.points[t], out.warp_confidence[t],
-                                                                  d_results->target_counts[t], (int)M);
-            CK(cudaGetLastError());
-            if (debug && debug->decision_kind) download(ctx, debug->decision_kind + (size_t)t * M, dec3.kind, M);
+            w.decisions[v] = p.out[v];
+            w.points[v] = out.points[t];
+            w.confidence[v] = out.warp_confidence[t];
+            w.counts[v] = d_results->target_counts[t];
             rewritten.push_back(t);
         }
+        warp_consensus_kernel<<<dim3(blocks_for(M, 256), V), 256, 0, s>>>(w);
+        warp_output_kernel<<<dim3(blocks_for(M, 256), V), 256, 0, s>>>(w);
+        CK(cudaGetLastError());
+        if (w.kinds)
+            for (int v = 0; v < V; ++v) download(ctx, debug->decision_kind + (size_t)targets[v] * M, w.kinds + (size_t)v * M, M);
     }
     record_event(ctx->events[6], s, capturing);
     if (capturing) {
@@ -2169,8 +2107,7 @@ int refine(chiaro_depth_ctx *ctx, const chiaro_view *views, size_t n_views, size
             }
             h_views[i] = dev_view(v, luma, pts);
         }
-        DevView *d_views = dbuf<DevView>(ctx, "views", n_views);
-        upload(ctx, d_views, h_views.data(), n_views);
+        DevView *d_views = dbuf<DevView>(ctx, "views", n_views);  // filled by the stage
         StageOutputs out{};
         if (device_pointers) {
             out.depth = out_map->depth;
@@ -2581,7 +2518,7 @@ int chiaro_warp_decisions_filter(chiaro_depth_ctx *ctx, uint8_t *kind, float *gl
         CK(cudaSetDevice(ctx->device));
         size_t n = columns * rows;
         cudaStream_t s = ctx->stream;
-        Decisions a = decision_bufs(ctx, "op.dec", n), b = decision_bufs(ctx, "op.dec2", n);
+        Decisions a = decision_bufs(ctx, "op.dec", n);
         float *dg = dbuf<float>(ctx, "op.guid", n);
         upload(ctx, a.kind, kind, n);
         upload(ctx, a.global, reinterpret_cast<const float2 *>(global), n);
@@ -2589,21 +2526,28 @@ int chiaro_warp_decisions_filter(chiaro_depth_ctx *ctx, uint8_t *kind, float *gl
         upload(ctx, a.measured, measured, n);
         CK(cudaMemsetAsync(a.confidence, 0, n * 4, s));
         upload(ctx, dg, guidance, n);
-        if (consensus) {
-            copy_decisions(ctx, b, a, n);
-            warp_consensus_kernel<<<blocks_for(n, 256), 256, 0, s>>>(a, b, (int)columns, (int)rows);
-            std::swap(a, b);
-        }
-        if (boundaries) {
-            copy_decisions(ctx, b, a, n);
-            warp_boundary_kernel<<<blocks_for(n, 256), 256, 0, s>>>(a, b, dg, (int)columns, (int)rows);
-            std::swap(a, b);
-        }
+        WarpPasses w{};
+        w.decisions[0] = a;
+        w.agreed = dbuf<uint8_t>(ctx, "op.agreed", n);
+        w.kinds = dbuf<uint8_t>(ctx, "op.kinds", n);
+        w.guidance = dg;
+        w.columns = (int)columns;
+        w.rows = (int)rows;
+        if (consensus)
+            warp_consensus_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w);
+        else
+            CK(cudaMemcpyAsync(w.agreed, a.kind, n, cudaMemcpyDeviceToDevice, s));
+        if (boundaries) warp_output_kernel<<<blocks_for(n, 256), 256, 0, s>>>(w);
         CK(cudaGetLastError());
-        download(ctx, kind, a.kind, n);
-        download(ctx, reinterpret_cast<float2 *>(global), a.global, n);
-        download(ctx, reinterpret_cast<float2 *>(point), a.point, n);
+        const std::vector<uint8_t> before(kind, kind + n);
+        download(ctx, kind, boundaries ? w.kinds : w.agreed, n);
         CK(cudaStreamSynchronize(s));
+        // an overruled node's point is its global mapping
+        for (size_t i = 0; i < n; ++i)
+            if (kind[i] != before[i]) {
+                point[2 * i] = global[2 * i];
+                point[2 * i + 1] = global[2 * i + 1];
+            }
     } catch (const CudaError &e) {
         return fail(ctx, e);
     }
