@@ -53,7 +53,7 @@ struct CostParams {
     TapLattice lattice;         // of this grid, or planes == nullptr
     int minimum_support, best_view_count;
     float *view_scores;         // scratch [CTA][tile nodes][target][slot] of the launch
-    double2 *places;            // scratch [CTA][tile nodes * slots]
+    double2 *places;            // scratch [CTA (x, then y)][tile nodes * slots]
     float *scores, *costs, *guidance;
     uint8_t *tested;
     // label subsets (slots == labels with no list and no bands: the full volume)
@@ -130,6 +130,75 @@ __device__ inline TileSmem carve_tile_smem(unsigned char *base, int K, int taps,
 
 constexpr int TILE_NODES = 8;  // most nodes of a CTA
 
+// Node k of a tile CTA (-1: none) and its output row: consecutive entries of a node list, or a
+// block of the grid.
+__device__ __forceinline__ int tile_node(const CostParams &p, int n_rows, int k, int &row) {
+    if (p.node_list) {
+        row = blockIdx.x * p.tile_w * p.tile_h + k;
+        return row < n_rows ? __ldg(p.node_list + row) : -1;
+    }
+    const int tiles_x = (p.columns + p.tile_w - 1) / p.tile_w, ty = blockIdx.x / tiles_x;
+    const int r = ty * p.tile_h + k / p.tile_w, c = (blockIdx.x - ty * tiles_x) * p.tile_w + k % p.tile_w;
+    row = r * p.columns + c;
+    return r < p.rows && c < p.columns ? row : -1;
+}
+
+// Aggregates the views per label of a tile's nodes and prices the labels (depth.rs:1233-1246);
+// every thread of the CTA. score: [K][V][D].
+__device__ inline void aggregate_tile(const CostParams &p, const float *score, const int *node_of, const int *row_of,
+                                      int *tested) {
+    const int K = p.tile_w * p.tile_h, V = p.n_targets, D = p.slots;
+    const SmallDiv by_slots(D);
+    if (threadIdx.x < K) tested[threadIdx.x] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < K * D; i += blockDim.x) {
+        const int k = by_slots.quotient(i), slot = i - k * D, node = node_of[k];
+        if (node < 0) continue;
+        const int label = cost_slot_label(p, node, slot);
+        const float *views = score + k * V * D + slot;
+        float agg = 0.0f;
+        bool some;
+        if (V <= 4) {  // the views' scores in registers (V is the same for the whole launch)
+            some = aggregate_small<4>(views, D, V, p.minimum_support, p.best_view_count, agg);
+        } else if (V <= 8) {
+            some = aggregate_small<8>(views, D, V, p.minimum_support, p.best_view_count, agg);
+        } else {
+            float sc[MAX_VIEWS];
+            for (int v = 0; v < V; ++v) sc[v] = views[v * D];
+            some = aggregate_scores(sc, V, p.minimum_support, p.best_view_count, agg);
+        }
+        const float total = some ? agg : NAN;
+        float cost;
+        if (isfinite(total)) {
+            tested[k] = 1;
+            float near_prior = label == 0 ? 0.0f : NEAR_DEPTH_PRIOR * (float)(label - 1) / (float)(p.labels - 2);
+            cost = clampf_r(1.0f - total, 0.0f, 2.0f) + near_prior;
+        } else {
+            cost = MISSING_COST;
+        }
+        const size_t o = (size_t)row_of[k] * D + slot;
+        p.scores[o] = total;
+        p.costs[o] = cost;
+    }
+    __syncthreads();
+    if (threadIdx.x < K && node_of[threadIdx.x] >= 0) {
+        p.tested[row_of[threadIdx.x]] = (uint8_t)tested[threadIdx.x];
+        // reference_guidance (depth.rs:1824-1832)
+        p.guidance[row_of[threadIdx.x]] = p.patches[node_of[threadIdx.x]].centre;
+    }
+}
+
+// The aggregation of a launch whose CTAs scored one target each.
+__global__ void __launch_bounds__(128) cost_aggregate_kernel(CostParams p, int n_rows) {
+    __shared__ int node_of[TILE_NODES], row_of[TILE_NODES], tested[TILE_NODES];
+    const int K = p.tile_w * p.tile_h;
+    if (threadIdx.x < K) node_of[threadIdx.x] = tile_node(p, n_rows, threadIdx.x, row_of[threadIdx.x]);
+    aggregate_tile(p, p.view_scores + (size_t)blockIdx.x * K * p.n_targets * p.slots, node_of, row_of, tested);
+}
+
+// A CTA scores its tile for every target in turn and aggregates; where the grid is so small that
+// the targets' turns are the launch's latency, it scores target blockIdx.y alone and
+// cost_aggregate_kernel follows (gridDim.y > 1).
 // Registers bounded to 64 per thread at every shape (1024 / T CTAs per SM).
 template <int T>
 __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, int n_rows) {
@@ -147,30 +216,21 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int warps = T / 32;
-    const int K = p.tile_w * p.tile_h, V = p.n_targets, D = p.slots, full_labels = p.labels;
+    const int K = p.tile_w * p.tile_h, V = p.n_targets, D = p.slots;
     const int side = 2 * p.radius + 1, taps = side * side, pairs = (taps + 1) / 2;
     const SmallDiv by_slots(D), by_pairs(pairs);
     const TileSmem s = carve_tile_smem(smem_raw, K, taps, D, p.region_rows);
     float *const score = p.view_scores + (size_t)blockIdx.x * K * V * D;  // [K][V][D], NaN = None
-    double2 *const places = p.places + (size_t)blockIdx.x * K * D;         // displacements of the list's back
+    // displacements of the list's back
+    double2 *const places = p.places + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * K * D;
     const DevView &rv = p.views[p.reference];
     const TapLattice &lat = p.lattice;
 
-    // ---- the tile's nodes: consecutive entries of a node list, or a block of the grid
     if (tid < K) {
-        int node = -1, row = -1;
-        if (p.node_list) {
-            row = blockIdx.x * K + tid;
-            if (row < n_rows) node = __ldg(p.node_list + row);
-        } else {
-            const int tiles_x = (p.columns + p.tile_w - 1) / p.tile_w;
-            const int ty = blockIdx.x / tiles_x, tx = blockIdx.x - ty * tiles_x;
-            const int r = ty * p.tile_h + tid / p.tile_w, c = tx * p.tile_w + tid % p.tile_w;
-            if (r < p.rows && c < p.columns) row = node = r * p.columns + c;
-        }
+        int row;
+        const int node = tile_node(p, n_rows, tid, row);
         node_of[tid] = node;
         row_of[tid] = row;
-        tested[tid] = 0;
         if (node >= 0) {
             patch[tid] = p.patches[node];
             if (lat.planes)
@@ -205,7 +265,8 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
         s.weight[i] = make_float4(w[0], w[1], wr[0], wr[1]);
     }
 
-    for (int v = 0; v < V; ++v) {
+    const int first_target = gridDim.y > 1 ? blockIdx.y : 0, end_target = gridDim.y > 1 ? first_target + 1 : V;
+    for (int v = first_target; v < end_target; ++v) {
         const DevView &tv = p.views[p.targets[v]];
         __syncthreads();  // the weights, or the last target's correlations
         for (int i = tid; i < (int)(sizeof(DevCamera) / 8); i += T)
@@ -357,43 +418,259 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
             if (pass + 1 < passes) __syncthreads();  // the list and the region are written again
         }
     }
+    if (gridDim.y > 1) return;
+    __syncthreads();
+    aggregate_tile(p, score, node_of, row_of, tested);
+}
+
+// Dynamic shared memory of a node CTA.
+struct NodeSmem {
+    ViewGeom *geom;        // [V]
+    TapBox *box;           // [V]
+    float *rr;             // [T] (w r) r
+    float2 *wt;            // [T] (w, w r)
+    double2 *gh;           // [V][T] g/2 of the tap positions
+    float *score;          // [V][D] per-view scores, NaN = None
+    unsigned short *list;  // [V][D] scored items: fast path from the front, exact path from the back
+    double2 *disp;         // [V][D] displacement (ddx, ddy) of each item; ddx NaN: out of reach
+};
+
+__host__ __device__ inline size_t node_form_bytes(int V, int taps, int labels) {
+    const size_t items = (size_t)V * labels;
+    return align16(V * sizeof(ViewGeom)) + align16(V * sizeof(TapBox)) + align16(taps * sizeof(float)) +
+           align16(taps * sizeof(float2)) + align16((size_t)V * taps * sizeof(double2)) +
+           align16(items * sizeof(float)) + align16(items * sizeof(unsigned short)) + items * sizeof(double2);
+}
+
+__device__ inline NodeSmem carve_node_smem(unsigned char *base, int V, int taps, int labels) {
+    const size_t items = (size_t)V * labels;
+    NodeSmem s;
+    size_t o = 0;
+    s.geom = reinterpret_cast<ViewGeom *>(base + o);
+    o += align16(V * sizeof(ViewGeom));
+    s.box = reinterpret_cast<TapBox *>(base + o);
+    o += align16(V * sizeof(TapBox));
+    s.rr = reinterpret_cast<float *>(base + o);
+    o += align16(taps * sizeof(float));
+    s.wt = reinterpret_cast<float2 *>(base + o);
+    o += align16(taps * sizeof(float2));
+    s.gh = reinterpret_cast<double2 *>(base + o);
+    o += align16((size_t)V * taps * sizeof(double2));
+    s.score = reinterpret_cast<float *>(base + o);
+    o += align16(items * sizeof(float));
+    s.list = reinterpret_cast<unsigned short *>(base + o);
+    o += align16(items * sizeof(unsigned short));
+    s.disp = reinterpret_cast<double2 *>(base + o);
+    return s;
+}
+
+// The form for small planes: a CTA per node, every target's items at once, samples gathered from
+// the quad plane in f64. A plane of a few hundred pixels has most of its patches near an edge,
+// where the f32 positions do not hold, and its grid is a wave or two of CTAs, whose latency
+// counts: there a tile's turns cost more than its shared samples give (coarse search, node / tile:
+// 342x249 with five targets 62 / 87 us, 363x288 with four 187 / 232 us, 569x342 with four 216 / 231;
+// 778x528 with five 154 / 154, 966x661 with three 98 / 84, 1041x764 with three 752 / 662).
+constexpr int COST_TILE_SIDE = 320;  // the largest target side (of the luminance plane) from which tiles pay
+
+template <int T>
+__global__ void __launch_bounds__(T, 1024 / T) cost_volume_node_kernel(CostParams p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ RefPatch patch;
+    __shared__ unsigned warp_undefined[T / 32];  // bit v: a tap of target v has no global warp
+    __shared__ int list_ends[2];                 // fast items listed, exact items listed
+    const unsigned full = 0xffffffffu;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int warps = T / 32;
+    const int out_row = blockIdx.x;
+    const int node = p.node_list ? __ldg(p.node_list + out_row) : out_row;
+    const int V = p.n_targets, D = p.slots, full_labels = p.labels;
+    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
+    const int total = V * D;
+    const int chunks = (total + T - 1) / T;
+    const SmallDiv by_slots(D), by_taps(taps), side(2 * p.radius + 1);  // item / D, i / taps, tap rows
+    NodeSmem s = carve_node_smem(smem_raw, V, taps, D);
+    const double cx = (double)((node % p.columns) * p.step), cy = (double)((node / p.columns) * p.step);
+    const DevView &rv = p.views[p.reference];
+    const D3 origin = camera_origin(rv.cam);
+
+    // ---- staging: geometry, reference patch, tap positions (from the tap lattice when
+    // the grid has one)
+    if (tid < V) geom_from_rec(p.geometry[(size_t)node * V + tid], origin, s.geom[tid]);
+    if (tid < 2) list_ends[tid] = 0;  // read after the staging's barriers
+    const TapLattice &lat = p.lattice;
+    const size_t at0 = lat.planes ? lat.index(cx, cy) : 0;
+    float centre = 0.0f;
+    bool centre_ok;
+    if (lat.planes) {
+        const float2 c = __ldg(lat.planes + at0);
+        centre = c.x;
+        centre_ok = c.y != 0.0f;
+    } else {
+        centre_ok = plane_sample(rv.luma, (float)((cx - 0.5) * 0.5), (float)((cy - 0.5) * 0.5), centre);
+    }
+    bool sampled = true;
+    for (int t = tid; t < taps; t += T) {
+        int dx, dy;
+        tap_offset(t, p.radius, side, dx, dy);
+        float value = 0.0f;
+        if (lat.planes) {
+            const float2 r = __ldg(lat.planes + at0 + (ptrdiff_t)dy * lat.columns + dx);
+            value = r.x;
+            sampled &= r.y != 0.0f;
+        } else {
+            double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
+            sampled &= plane_sample(rv.luma, (float)((px - 0.5) * 0.5), (float)((py - 0.5) * 0.5), value);
+        }
+        float weight = p.spatial[t] * exp_f32(-1.2f * fabsf(value - centre));
+        float weighted = weight * value;
+        s.wt[t] = make_float2(weight, weighted);
+        s.rr[t] = weighted * value;
+    }
+    unsigned undefined = 0u;
+    for (int i = tid; i < V * taps; i += T) {
+        const int v = by_taps.quotient(i), t = i - v * taps;
+        int dx, dy;
+        tap_offset(t, p.radius, side, dx, dy);
+        float qx = 0.0f, qy = 0.0f;
+        if (lat.planes) {
+            const float2 q = __ldg(lat.planes + (size_t)(v + 1) * lat.plane_size() + at0 +
+                                   (ptrdiff_t)dy * lat.columns + dx);
+            qx = q.x;
+            qy = q.y;
+            if (qx != qx) undefined |= 1u << v;
+        } else {
+            double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
+            if (!warp_map(p.views[p.targets[v]].warp, (float)px, (float)py, qx, qy)) undefined |= 1u << v;
+        }
+        store_tap(s.gh[i], qx, qy);
+    }
+    undefined = __reduce_or_sync(full, undefined);
+    if (lane == 0) warp_undefined[warp] = undefined;
+    const bool all_sampled = __syncthreads_and(sampled);
+    // displacement of every (target, slot) item, view-major: item = v * D + slot
+    for (int item = tid; item < total; item += T) {
+        const int v = by_slots.quotient(item), label = cost_slot_label(p, node, item - v * D);
+        const ViewGeom &g = s.geom[v];
+        double ddx = 0.0, ddy = 0.0;
+        bool ok = g.gc_ok;
+        if (ok && label > 0) ok = depth_delta(p.views[p.targets[v]].cam, g, p.label_depth[label], ddx, ddy);
+        s.disp[item] = make_double2(ok ? ddx : NAN, ddy);
+    }
+    // tap boxes (eight lanes per target) and the three sequential reference
+    // sums (lanes 0-2 of the warp after the box warps)
+    for (int vb = warp * 4; vb < V; vb += 4 * warps) {
+        const int v = vb + (lane >> 3);
+        TapBox b = group8_tap_box(s.gh + (v < V ? v : V - 1) * taps, taps);
+        if ((lane & 7) == 0 && v < V) s.box[v] = b;
+    }
+    if (warp == ((V + 3) / 4) % warps) {
+        float sum = 0.0f;
+        if (lane < 3)
+            sum = lane == 2 ? sequential_sum(s.rr, 1, taps)
+                            : sequential_sum(reinterpret_cast<const float *>(s.wt) + lane, 2, taps);
+        const float count = __shfl_sync(full, sum, 0), sum_r = __shfl_sync(full, sum, 1);
+        const float sum_rr = __shfl_sync(full, sum, 2);
+        if (lane == 0) {
+            patch.count = count;
+            patch.sum_r = sum_r;
+            patch.sum_rr = sum_rr;
+            patch.ref_energy = sum_rr - sum_r * sum_r / count;
+            patch.centre = centre;
+            patch.ok = centre_ok && all_sampled;
+        }
+    }
+    __syncthreads();
+
+    // ---- which items are scored, and on which path; then list them: fast ones from the
+    // front, exact ones from the back. A warp reserves its chunk's places at either end with
+    // one shared atomic add each; the order of the list only decides which thread scores
+    // which item (each score is computed alone into its own slot), so it does not change
+    // a result.
+    const bool patch_ok = patch.ok;
+    unsigned taps_bad = 0u;
+    for (int w = 0; w < warps; ++w) taps_bad |= warp_undefined[w];
+    const unsigned below = (1u << lane) - 1u;
+    for (int c = 0; c < chunks; ++c) {
+        const int item = c * T + tid;
+        bool scored = false, fast = false;
+        if (item < total) {
+            const int v = by_slots.quotient(item);
+            const double2 dd = s.disp[item];
+            scored = !(dd.x != dd.x) && patch_ok && !((taps_bad >> v) & 1u);
+            if (scored) {
+                const PlaneRef &plane = p.views[p.targets[v]].luma;
+                fast = taps_inside(tap_range(s.box[v], dd.x * 0.5, dd.y * 0.5), plane.width, plane.height);
+            } else {
+                s.score[item] = NAN;
+            }
+        }
+        const unsigned fast_mask = __ballot_sync(full, scored && fast);
+        const unsigned exact_mask = __ballot_sync(full, scored && !fast);
+        int fast_at = 0, exact_at = 0;
+        if (lane == 0) {
+            if (fast_mask) fast_at = atomicAdd(&list_ends[0], __popc(fast_mask));
+            if (exact_mask) exact_at = atomicAdd(&list_ends[1], __popc(exact_mask));
+        }
+        fast_at = __shfl_sync(full, fast_at, 0);
+        exact_at = __shfl_sync(full, exact_at, 0);
+        if (scored && fast) s.list[fast_at + __popc(fast_mask & below)] = (unsigned short)item;
+        if (scored && !fast) s.list[total - 1 - (exact_at + __popc(exact_mask & below))] = (unsigned short)item;
+    }
+    __syncthreads();
+    const int n_fast = list_ends[0], n_exact = list_ends[1];
+
+    // ---- the correlations of the listed items; an item's path is known from its place
+    const int listed = n_fast + n_exact;
+    for (int j = tid; j < listed; j += T) {
+        const bool fast = j < n_fast;
+        const int item = s.list[fast ? j : total - 1 - (j - n_fast)];
+        const int v = by_slots.quotient(item);
+        const DevView &tv = p.views[p.targets[v]];
+        const double2 dd = s.disp[item];
+        float score;
+        bool ok;
+        if (fast)
+            score = zncc_inside<9>(tv.quads, tv.quad_stride, s.gh + v * taps, s.wt, patch, taps, dd.x * 0.5, dd.y * 0.5,
+                                   ok);
+        else
+            ok = zncc_score(tv.luma, s.gh + v * taps, s.wt, patch, taps, dd.x, dd.y, score);
+        s.score[item] = ok ? score : NAN;
+    }
     __syncthreads();
 
     // ---- aggregate the views per label and price the label (depth.rs:1233-1246)
-    for (int i = tid; i < K * D; i += T) {
-        const int k = by_slots.quotient(i), slot = i - k * D, node = node_of[k];
-        if (node < 0) continue;
+    int any_finite = 0;
+    for (int slot = tid; slot < D; slot += T) {
         const int label = cost_slot_label(p, node, slot);
-        const float *views = score + k * V * D + slot;
         float agg = 0.0f;
         bool some;
         if (V <= 4) {  // the views' scores in registers (V is the same for the whole launch)
-            some = aggregate_small<4>(views, D, V, p.minimum_support, p.best_view_count, agg);
+            some = aggregate_small<4>(s.score + slot, D, V, p.minimum_support, p.best_view_count, agg);
         } else if (V <= 8) {
-            some = aggregate_small<8>(views, D, V, p.minimum_support, p.best_view_count, agg);
+            some = aggregate_small<8>(s.score + slot, D, V, p.minimum_support, p.best_view_count, agg);
         } else {
             float sc[MAX_VIEWS];
-            for (int v = 0; v < V; ++v) sc[v] = views[v * D];
+            for (int v = 0; v < V; ++v) sc[v] = s.score[v * D + slot];
             some = aggregate_scores(sc, V, p.minimum_support, p.best_view_count, agg);
         }
-        const float total = some ? agg : NAN;
+        float score = some ? agg : NAN;
         float cost;
-        if (isfinite(total)) {
-            tested[k] = 1;
+        if (isfinite(score)) {
+            any_finite = 1;
             float near_prior =
                 label == 0 ? 0.0f : NEAR_DEPTH_PRIOR * (float)(label - 1) / (float)(full_labels - 2);
-            cost = clampf_r(1.0f - total, 0.0f, 2.0f) + near_prior;
+            cost = clampf_r(1.0f - score, 0.0f, 2.0f) + near_prior;
         } else {
             cost = MISSING_COST;
         }
-        const size_t o = (size_t)row_of[k] * D + slot;
-        p.scores[o] = total;
+        size_t o = (size_t)out_row * D + slot;
+        p.scores[o] = score;
         p.costs[o] = cost;
     }
-    __syncthreads();
-    if (tid < K && node_of[tid] >= 0) {
-        p.tested[row_of[tid]] = (uint8_t)tested[tid];
-        p.guidance[row_of[tid]] = patch[tid].centre;  // reference_guidance (depth.rs:1824-1832)
+    const bool tested = __syncthreads_or(any_finite);
+    if (tid == 0) {
+        p.tested[out_row] = tested;
+        p.guidance[out_row] = patch.centre;  // reference_guidance (depth.rs:1824-1832)
     }
 }
 

@@ -198,31 +198,33 @@ void download(chiaro_depth_ctx *ctx, T *dst, const T *src, size_t count) {
     CK(cudaMemcpyAsync(dst, src, count * sizeof(T), cudaMemcpyDeviceToHost, ctx->stream));
 }
 
-// Opt the kernels that need more than 48 KiB of dynamic shared memory in, once per
-// device (the attribute belongs to the current device's context).
-void set_smem_limits() {
-    static std::mutex lock;
-    static std::vector<int> done_devices;
-    int device = 0;
-    CK(cudaGetDevice(&device));
-    std::lock_guard<std::mutex> guard(lock);
-    if (std::find(done_devices.begin(), done_devices.end(), device) != done_devices.end()) return;
-    CK(cudaFuncSetAttribute(cost_volume_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(cost_volume_kernel<96>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(cost_volume_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(cost_volume_kernel<160>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(cost_volume_kernel<192>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false>,
-                        direct_wide_kernel<true>})
-        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(target_decision_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(target_decision_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(align_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    done_devices.push_back(device);
-}
-
 // ---- cost-volume launch shapes (the autotuner) -----------------------------------------
 typedef void (*CostKernel)(CostParams, int);
+typedef void (*CostNodeKernel)(CostParams);
+
+CostNodeKernel cost_node_kernel_for(int threads) {
+    switch (threads) {
+        case 64: return cost_volume_node_kernel<64>;
+        case 96: return cost_volume_node_kernel<96>;
+        case 160: return cost_volume_node_kernel<160>;
+        case 192: return cost_volume_node_kernel<192>;
+        default: return cost_volume_node_kernel<128>;
+    }
+}
+
+// Whether a full-range cost volume runs in node tiles (see COST_TILE_SIDE). The band search's
+// 17 and 25 labels a node do not fill a tile's turns (1888x1537, five targets: pre-pass 475 / 505
+// us, band 523 / 574 us, node / tile; 1100x803, three: 126 / 135, 142 / 142): they go node by node.
+// Below COST_TILE_ITEMS hypotheses the tiles' patch kernel costs what they save (723x531 with one
+// target and 65 labels, 0.41 M items: 81 -> 65 us and 15 us of set-up; 1040x780, 0.84 M: 310 -> 240).
+constexpr size_t COST_TILE_ITEMS = 600000;
+
+bool cost_in_tiles(const std::vector<DevView> &views, const std::vector<int> &targets, size_t nodes, int labels) {
+    if (nodes * targets.size() * labels < COST_TILE_ITEMS) return false;
+    int side = 0;
+    for (int t : targets) side = std::max({side, views[t].luma.width, views[t].luma.height});
+    return side >= COST_TILE_SIDE;
+}
 
 CostKernel cost_kernel_for(int threads) {
     switch (threads) {
@@ -232,6 +234,28 @@ CostKernel cost_kernel_for(int threads) {
         case 192: return cost_volume_kernel<192>;
         default: return cost_volume_kernel<128>;
     }
+}
+
+// Opt the kernels that need more than 48 KiB of dynamic shared memory in, once per
+// device (the attribute belongs to the current device's context).
+void set_smem_limits() {
+    static std::mutex lock;
+    static std::vector<int> done_devices;
+    int device = 0;
+    CK(cudaGetDevice(&device));
+    std::lock_guard<std::mutex> guard(lock);
+    if (std::find(done_devices.begin(), done_devices.end(), device) != done_devices.end()) return;
+    for (int threads : COST_SHAPES) {
+        CK(cudaFuncSetAttribute(cost_kernel_for(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        CK(cudaFuncSetAttribute(cost_node_kernel_for(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    }
+    for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false>,
+                        direct_wide_kernel<true>})
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(target_decision_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(target_decision_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    CK(cudaFuncSetAttribute(align_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    done_devices.push_back(device);
 }
 
 // The tile, the region buffer and each target's axis and passes for a cost-volume launch.
@@ -258,7 +282,9 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
         p.tile_h = p.node_list ? 1 : shape[1];
         if (nodes == 8 && (p.slots > 80 || n_rows < (size_t)16 * nodes * sm_count) && p.slots > 32)
             continue;  // four nodes fill the CTA's threads
-        if (n_rows < (size_t)nodes * 4 * sm_count) continue;  // a small grid: more CTAs instead
+        if (nodes > 4 && (p.tile_w - 1) * p.step / 2 + 64 + 2 * p.radius + 11 > REGION_PITCH)
+            continue;  // its samples would not fit a row of the region
+        if (n_rows * std::max(p.n_targets, 1) < (size_t)nodes * 4 * sm_count) continue;  // a small grid: more CTAs instead
         if (tile_smem_bytes(nodes, taps, p.slots, p.region_rows) <= 56 * 1024) break;
     }
     const DevView &rv = views[p.reference];
@@ -300,16 +326,31 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
 void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView> &views, size_t n_rows,
                  size_t path_floats) {
     cudaStream_t s = ctx->stream;
-    plan_cost_tiles(p, views, n_rows, ctx->sm_count);
-    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1), nodes = p.tile_w * p.tile_h;
-    const size_t smem = tile_smem_bytes(nodes, taps, p.slots, p.region_rows);
-    const unsigned blocks = (unsigned)(p.node_list ? div_ceil(n_rows, nodes)
-                                                   : div_ceil(p.columns, p.tile_w) * div_ceil(p.rows, p.tile_h));
-    // the launch's scratch shares the SGM's path buffers, which are free until the volume is done
-    const size_t items = (size_t)blocks * nodes * p.slots;
-    float *scratch = dbuf<float>(ctx, "sgm_paths", std::max(items * (4 + p.n_targets), path_floats));
-    p.places = reinterpret_cast<double2 *>(scratch);
-    p.view_scores = scratch + 4 * items;
+    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
+    const bool tiles = p.patches != nullptr;
+    size_t smem = node_form_bytes(p.n_targets, taps, p.slots);
+    unsigned blocks = (unsigned)n_rows, turns = 1;
+    if (tiles) {
+        plan_cost_tiles(p, views, n_rows, ctx->sm_count);
+        const int nodes = p.tile_w * p.tile_h;
+        smem = tile_smem_bytes(nodes, taps, p.slots, p.region_rows);
+        blocks = (unsigned)(p.node_list ? div_ceil(n_rows, nodes)
+                                        : div_ceil(p.columns, p.tile_w) * div_ceil(p.rows, p.tile_h));
+        // a grid of less than two waves of CTAs (seven an SM): a CTA per target
+        if (p.n_targets > 1 && blocks < 14u * ctx->sm_count) turns = (unsigned)p.n_targets;
+        // the launch's scratch shares the SGM's path buffers, which are free until the volume is done
+        const size_t items = (size_t)blocks * nodes * p.slots;
+        float *scratch = dbuf<float>(ctx, "sgm_paths", std::max(items * (4 * turns + p.n_targets), path_floats));
+        p.places = reinterpret_cast<double2 *>(scratch);
+        p.view_scores = scratch + 4 * items * turns;
+    }
+    const auto launch = [&](int threads) {
+        if (tiles)
+            cost_kernel_for(threads)<<<dim3(blocks, turns), threads, smem, s>>>(p, (int)n_rows);
+        else
+            cost_node_kernel_for(threads)<<<blocks, threads, smem, s>>>(p);
+        CK(cudaGetLastError());
+    };
     const uint64_t key = ((uint64_t)p.n_targets << 24) | ((uint64_t)p.slots << 8) | (uint64_t)p.radius;
     int threads = ctx->autotune > 1 ? ctx->autotune : COST_THREADS;
     auto it = ctx->cost_tuning.find(key);
@@ -328,8 +369,7 @@ void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView>
             float ms = 0.0f;
             for (int rep = 0; rep < 2; ++rep) {
                 CK(cudaEventRecord(e0, s));
-                cost_kernel_for(t)<<<blocks, t, smem, s>>>(p, (int)n_rows);
-                CK(cudaGetLastError());
+                launch(t);
                 CK(cudaEventRecord(e1, s));
                 CK(cudaEventSynchronize(e1));
                 CK(cudaEventElapsedTime(&ms, e0, e1));
@@ -343,8 +383,12 @@ void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView>
         cudaEventDestroy(e1);
         ctx->cost_tuning[key] = threads;
     }
-    cost_kernel_for(threads)<<<blocks, threads, smem, s>>>(p, (int)n_rows);
-    CK(cudaGetLastError());
+    launch(threads);
+    if (turns > 1) {
+        cost_aggregate_kernel<<<blocks, 128, 0, s>>>(p, (int)n_rows);
+        CK(cudaGetLastError());
+        ctx->launches += 1;
+    }
 }
 
 // Per (node, target) geometry records of one or two step-spaced grids.
@@ -1261,8 +1305,12 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     }
     launch_sample_planes(ctx, g.views, h_views, g.targets);
     g.h_views = h_views;
-    g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
-    launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
+    const auto full_range_patches = [&] {  // the node tiles of a full-range cost volume read them
+        if (!cost_in_tiles(h_views, g.targets, N, D)) return;
+        g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
+        launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
+    };
+    if (!spec) full_range_patches();
     CK(cudaEventRecord(ctx->events[1], s));
     uint8_t *tested = dbuf<uint8_t>(ctx, "coarse.tested", N);
     float *guidance = dbuf<float>(ctx, "coarse.guidance", N);
@@ -1378,6 +1426,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
             float *wguid = dbuf<float>(ctx, "coarse.window_guidance", node_count);
             uint8_t *wtested = dbuf<uint8_t>(ctx, "coarse.window_tested", node_count);
             float *wagg = dbuf<float>(ctx, "coarse.window_aggregate", cost_floats);
+            full_range_patches();
             coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, d_nodes, node_count, wscores, wcosts, wguid,
                         wtested);
             if (windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows) {
@@ -1703,12 +1752,15 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     // each fine node's reference patch at the direct radius, read by the direct pass and,
     // at the same radius, by the decisions
     RefPatch *fine_patches = dbuf<RefPatch>(ctx, "fine_patches", M);
-    RefPatch *coarse_patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
-    launch_patches(ctx, d_views, reference,
-                   {{(int)g.columns, (int)g.rows, (int)g.step, direct_radius, d_sp_direct,
-                     fine_lattice ? lattice : TapLattice{}, fine_patches},
-                    {(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, radius, d_sp,
-                     coarse_lattice ? lattice : TapLattice{}, coarse_patches}});
+    RefPatch *coarse_patches = nullptr;  // the node tiles of the cost volume read them
+    std::vector<PatchGrid> patch_grids{{(int)g.columns, (int)g.rows, (int)g.step, direct_radius, d_sp_direct,
+                                        fine_lattice ? lattice : TapLattice{}, fine_patches}};
+    if (cost_in_tiles(h_views, targets, N, D)) {
+        coarse_patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
+        patch_grids.push_back({(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, radius, d_sp,
+                               coarse_lattice ? lattice : TapLattice{}, coarse_patches});
+    }
+    launch_patches(ctx, d_views, reference, patch_grids);
     if (host_planes) CK(cudaStreamWaitEvent(s, ctx->planes_ready, 0));
     // quad planes of the target luminance for the fast ZNCC path
     launch_sample_planes(ctx, d_views, h_views, targets);

@@ -122,6 +122,7 @@ __device__ inline TapBox group8_tap_box(const TapT *gh, int taps) {
 // patch sums add w, w r and (w r) r tap by tap).
 __device__ inline float sequential_sum(const float *a, int stride, int taps) {
     float sum = 0.0f;
+#pragma unroll 9
     for (int t = 0; t < taps; ++t) sum += a[t * stride];
     return sum;
 }
@@ -288,7 +289,6 @@ __global__ void __launch_bounds__(256) patch_sums_kernel(PatchParams params) {
     const double cx = (double)((int)(i % p.columns) * p.step), cy = (double)((int)(i / p.columns) * p.step);
     const DevView &rv = params.views[params.reference];
     const TapLattice &lattice = p.lattice;
-    const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
     float centre = 0.0f;
     bool centre_ok;
     const size_t at0 = lattice.planes ? lattice.index(cx, cy) : 0;
@@ -301,23 +301,46 @@ __global__ void __launch_bounds__(256) patch_sums_kernel(PatchParams params) {
     }
     bool sampled = true;
     float count = 0.0f, sum_r = 0.0f, sum_rr = 0.0f;
-    for (int t = 0; t < taps; ++t) {
-        int dx, dy;
-        tap_offset(t, p.radius, dx, dy);
-        float value = 0.0f;
+    // eight taps' loads and weights at a time, ahead of their sums: on a small grid the kernel is
+    // one thread's latency (27 us at 660 nodes with every tap's loads after the last one's sums)
+    constexpr int AHEAD = 8;
+    const int side = 2 * p.radius + 1, taps = side * side;
+    const SmallDiv by_side(side);
+    for (int t0 = 0; t0 < taps; t0 += AHEAD) {
+        float value[AHEAD], weight[AHEAD];
         if (lattice.planes) {
-            const float2 r = __ldg(lattice.planes + at0 + (ptrdiff_t)dy * lattice.columns + dx);
-            value = r.x;
-            sampled &= r.y != 0.0f;
+            float2 r[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                int dx, dy;
+                tap_offset(min(t0 + i, taps - 1), p.radius, by_side, dx, dy);
+                r[i] = __ldg(lattice.planes + at0 + (ptrdiff_t)dy * lattice.columns + dx);
+            }
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i) {
+                value[i] = r[i].x;
+                sampled &= r[i].y != 0.0f;
+            }
         } else {
-            double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
-            sampled &= plane_sample(rv.luma, (float)((px - 0.5) * 0.5), (float)((py - 0.5) * 0.5), value);
+            for (int i = 0; i < AHEAD; ++i) {
+                int dx, dy;
+                tap_offset(min(t0 + i, taps - 1), p.radius, by_side, dx, dy);
+                const double px = cx + (double)dx * 2.0, py = cy + (double)dy * 2.0;
+                value[i] = 0.0f;
+                sampled &= plane_sample(rv.luma, (float)((px - 0.5) * 0.5), (float)((py - 0.5) * 0.5), value[i]);
+            }
         }
-        float weight = __ldg(p.spatial + t) * exp_f32(-1.2f * fabsf(value - centre));
-        float weighted = weight * value;
-        count += weight;
-        sum_r += weighted;
-        sum_rr += weighted * value;
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            weight[i] = __ldg(p.spatial + min(t0 + i, taps - 1)) * exp_f32(-1.2f * fabsf(value[i] - centre));
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i)
+            if (t0 + i < taps) {
+                const float weighted = weight[i] * value[i];
+                count += weight[i];
+                sum_r += weighted;
+                sum_rr += weighted * value[i];
+            }
     }
     RefPatch r;
     r.count = count;

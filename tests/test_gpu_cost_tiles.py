@@ -1,8 +1,8 @@
 """The cost volume's node tiles against the oracle, bit for bit, where they can go wrong:
 grids that no tile divides, one node column or row, few and many labels (every tile size and
 labels scored in several parts), epipolar lines near either axis (samples stored by rows or by
-columns), an odd step (no tap lattice), a patch larger than the default, and a plane so small
-that most patches start near its left and top edges (the f64 sample positions)."""
+columns), an odd step (no tap lattice), a patch larger than the default, and planes so small
+that they take the form without tiles."""
 import numpy as np
 import pytest
 
@@ -19,6 +19,12 @@ CASES = {
     "odd step": dict(width=331, height=220, sources=3, planes=70, step=9, radius=3, focal=None),
     "long reach": dict(width=560, height=430, sources=4, planes=128, step=8, radius=4, focal=2400.0),
     "large patch": dict(width=400, height=300, sources=2, planes=20, step=12, radius=9, focal=1500.0),
+    # planes of at least 320 pixels and 600,000 hypotheses: node tiles
+    "tiles, one target": dict(width=851, height=662, sources=1, planes=80, step=8, radius=4, focal=None),
+    "tiles, odd step": dict(width=433, height=845, sources=3, planes=70, step=9, radius=3, focal=None),
+    "tiles, long reach": dict(width=700, height=500, sources=4, planes=128, step=8, radius=4, focal=2400.0),
+    "tiles, fine grid": dict(width=642, height=480, sources=2, planes=30, step=4, radius=2, focal=1500.0),
+    "tiles, large patch": dict(width=640, height=400, sources=3, planes=110, step=12, radius=9, focal=1500.0),
 }
 
 
