@@ -17,6 +17,7 @@
 namespace chiaro {
 
 constexpr int MAX_DIRECT_CANDIDATES = 32;
+constexpr int WIDE_CANDIDATES = 7;  // of the wide retry: the best one and three on each side
 constexpr int KEY_NONE = -2147483647 - 1;  // below every total_key of a non-NaN float
 
 // select_direct_depth (depth.rs:1109-1165) and best_depth_candidate
@@ -100,30 +101,46 @@ struct DirectParams {
     Field out;
     float *guidance;
     uint8_t *tested;
-    int *wide_count;                                   // wide-retry list length
+    int *wide_count;                                   // wide-retry list length; entries taken beyond the first ones
     int4 *wide_list;                                   // (node, first, last, seeded)
 };
 
-// Per-warp shared memory of the direct pass for V targets and T taps; TapT
-// is the tap storage (load_tap).
+// Per-warp shared memory of the direct pass for V targets, T taps and up to `most` candidates;
+// TapT is the tap storage (load_tap; NoTap: they are read from the lattice).
 template <typename TapT>
 struct DirectSlot {
-    float *rr;             // [T] (w r) r
     float2 *wt;            // [T] (w, w r)
     ViewGeom *geom;        // [V]
-    TapT *gh;              // [V][T] tap positions g/2
+    TapT *gh;              // [V][T] taps
     TapBox *box;           // [V]
     double *cand;          // [32]
-    float2 *items;         // [33][V] a listed item on the grid: its f32 offset, until it is scored;
+    float *rr;             // [T] (w r) r: until the patch is summed, where the following then lie
+    float2 *items;         // [V][most + 1] a listed item on the grid: its f32 offset, until it is scored;
                            // then the score in x (NaN = None)
-    float *agg;            // [33]: [0] baseline, [1 + c] candidates
-    unsigned short *list;  // [33][V] scored items: fast path from the front, exact path from the back
+    float *agg;            // [most + 1]: [0] baseline, [1 + c] candidates
+    unsigned short *list;  // [V][most + 1] scored items: fast path from the front, exact path from the back
 };
 
 template <typename TapT>
-__host__ __device__ inline size_t direct_slot_bytes(int V, int taps) {
+__host__ __device__ inline size_t tap_bytes(int V, int taps) {
+    return std::is_empty<TapT>::value ? 0 : align16((size_t)V * taps * sizeof(TapT));
+}
+
+template <typename TapT>
+__host__ __device__ inline size_t direct_slot_bytes(int V, int taps, int most) {
+    const size_t items = align16((size_t)(most + 1) * V * sizeof(float2)) + align16((most + 1) * sizeof(float)) +
+                         align16((size_t)(most + 1) * V * sizeof(unsigned short));
+    const size_t sums = align16(taps * sizeof(float));
+    return align16(taps * sizeof(float2)) + align16(V * sizeof(ViewGeom)) +
+           tap_bytes<TapT>(V, taps) + align16(V * sizeof(TapBox)) +
+           align16(MAX_DIRECT_CANDIDATES * sizeof(double)) + (items > sums ? items : sums);
+}
+
+// The bound on targets and radius that the direct pass accepts, for its patch and its wide one:
+// a node's weights, positions, sums and items apart.
+inline size_t direct_bound_bytes(int V, int taps) {
     return align16(taps * sizeof(float)) + align16(taps * sizeof(float2)) + align16(V * sizeof(ViewGeom)) +
-           align16((size_t)V * taps * sizeof(TapT)) + align16(V * sizeof(TapBox)) +
+           align16((size_t)V * taps * sizeof(float2)) + align16(V * sizeof(TapBox)) +
            align16(MAX_DIRECT_CANDIDATES * sizeof(double)) +
            align16((size_t)(MAX_DIRECT_CANDIDATES + 1) * V * sizeof(float2)) +
            align16((MAX_DIRECT_CANDIDATES + 1) * sizeof(float)) +
@@ -131,25 +148,24 @@ __host__ __device__ inline size_t direct_slot_bytes(int V, int taps) {
 }
 
 template <typename TapT>
-__device__ inline DirectSlot<TapT> carve_direct_slot(unsigned char *base, int V, int taps) {
+__device__ inline DirectSlot<TapT> carve_direct_slot(unsigned char *base, int V, int taps, int most) {
     DirectSlot<TapT> d;
     size_t o = 0;
-    d.rr = reinterpret_cast<float *>(base);
-    o += align16(taps * sizeof(float));
-    d.wt = reinterpret_cast<float2 *>(base + o);
+    d.wt = reinterpret_cast<float2 *>(base);
     o += align16(taps * sizeof(float2));
     d.geom = reinterpret_cast<ViewGeom *>(base + o);
     o += align16(V * sizeof(ViewGeom));
     d.gh = reinterpret_cast<TapT *>(base + o);
-    o += align16((size_t)V * taps * sizeof(TapT));
+    o += tap_bytes<TapT>(V, taps);
     d.box = reinterpret_cast<TapBox *>(base + o);
     o += align16(V * sizeof(TapBox));
     d.cand = reinterpret_cast<double *>(base + o);
     o += align16(MAX_DIRECT_CANDIDATES * sizeof(double));
+    d.rr = reinterpret_cast<float *>(base + o);
     d.items = reinterpret_cast<float2 *>(base + o);
-    o += align16((size_t)(MAX_DIRECT_CANDIDATES + 1) * V * sizeof(float2));
+    o += align16((size_t)(most + 1) * V * sizeof(float2));
     d.agg = reinterpret_cast<float *>(base + o);
-    o += align16((MAX_DIRECT_CANDIDATES + 1) * sizeof(float));
+    o += align16((most + 1) * sizeof(float));
     d.list = reinterpret_cast<unsigned short *>(base + o);
     return d;
 }
@@ -213,8 +229,8 @@ __device__ inline void warp_stage_node(const DirectParams &p, const DirectSlot<T
 }
 
 // Warp-cooperative listing of the baseline and candidates cand[0..n) over all
-// targets. Item i is (candidate i / V - 1, target i % V), candidate -1 being the
-// baseline. It settles which items reach the correlation and which of them are fast (on
+// targets. Item v (n + 1) + c + 1 is candidate c in target v, candidate -1 being the
+// baseline: neighbouring lanes sample one target. It settles which items reach the correlation and which of them are fast (on
 // the grid, their offset in d.items; without GRID, inside the plane), sets the others'
 // scores to None and lists the scored ones: fast from the front of d.list, the rest from the
 // back of its (n + 1) V entries. Every lane returns the two counts.
@@ -226,6 +242,7 @@ __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<
     const unsigned below = (1u << lane) - 1u;
     const int V = p.n_targets;
     const int total = (n + 1) * V;
+    const SmallDiv by_target(n + 1);
     const ViewGeom *geom = d.geom;
     n_fast = 0;
     n_exact = 0;
@@ -233,7 +250,7 @@ __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<
         const int item = base + lane;
         bool scored = false, fast = false;
         if (item < total) {
-            const int c = item / V - 1, v = item - (item / V) * V;
+            const int v = by_target.quotient(item), c = item - v * (n + 1) - 1;
             const ViewGeom &g = geom[v];
             double ddx = 0.0, ddy = 0.0;
             bool ok = g.gc_ok;
@@ -261,24 +278,32 @@ __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<
     }
 }
 
-// The correlation of one listed item (warp_direct_list) into d.items; one thread. `fast`:
-// listed as on the grid.
-template <bool GRID, typename TapT>
+// The taps of target v in a node's slot, the node at (cx, cy).
+template <typename TapT>
+__device__ __forceinline__ auto direct_taps(const DirectParams &p, const DirectSlot<TapT> &d, double cx, double cy, int v,
+                                            int radius) {
+    if constexpr (std::is_same<TapT, NoTap>::value)
+        return lattice_taps(p.lattice, cx, cy, v, radius);
+    else
+        return static_cast<const TapT *>(d.gh + v * (2 * radius + 1) * (2 * radius + 1));
+}
+
+// The correlation of one listed item (warp_direct_list) of `count` a target into d.items, with
+// its target's taps; one thread. `fast`: listed as on the grid.
+template <bool GRID, int UNROLL, typename TapT, typename Taps>
 __device__ __forceinline__ void direct_item_score(const DirectParams &p, const DirectSlot<TapT> &d,
-                                                  const RefPatch &patch, const double *cand, int item, bool fast,
-                                                  int taps) {
-    const int V = p.n_targets;
-    const int c = item / V - 1, v = item - (item / V) * V;
+                                                  const RefPatch &patch, const double *cand, int count, int item,
+                                                  int v, const Taps &tap, bool fast, int taps) {
+    const int c = item - v * count - 1;
     const DevView &tv = p.views[p.targets[v]];
     float score;
     bool ok;
     if (GRID && fast) {
-        score = zncc_grid<3>(tv.quads, tv.quad_stride, d.gh + v * taps, d.wt, patch, taps,
-                          d.items[item], ok);
+        score = zncc_grid<UNROLL>(tv.quads, tv.quad_stride, tap, d.wt, patch, taps, d.items[item], ok);
     } else {
         double ddx = 0.0, ddy = 0.0;
         if (c >= 0) depth_delta(tv.cam, d.geom[v], cand[c], ddx, ddy);
-        ok = zncc_any<GRID ? 3 : 9>(tv, d.gh + v * taps, d.box[v], d.wt, patch, taps, ddx, ddy, score);
+        ok = zncc_any<GRID ? UNROLL : 9>(tv, tap, d.box[v], d.wt, patch, taps, ddx, ddy, score);
     }
     d.items[item].x = ok ? score : NAN;
 }
@@ -290,7 +315,7 @@ __device__ inline void warp_direct_aggregate(const DirectParams &p, const Direct
     const int V = p.n_targets;
     for (int c = threadIdx.x & 31; c <= n; c += 32) {
         float sc[MAX_VIEWS];
-        for (int v = 0; v < V; ++v) sc[v] = d.items[c * V + v].x;
+        for (int v = 0; v < V; ++v) sc[v] = d.items[v * (n + 1) + c].x;
         float a;
         d.agg[c] = aggregate_scores(sc, V, p.minimum_support, p.best_view_count, a) ? a : NAN;
     }
@@ -300,9 +325,9 @@ __device__ inline void warp_direct_aggregate(const DirectParams &p, const Direct
 // Warp-cooperative scores of the baseline and candidates cand[0..n) over all
 // targets, aggregated into d.agg[0..n] (NaN = None): the node's list, scored by
 // its own warp.
-template <bool GRID, typename TapT>
+template <bool GRID, int UNROLL, typename TapT>
 __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlot<TapT> &d, const RefPatch &patch,
-                                          const double *cand, int n, int radius) {
+                                          const double *cand, int n, int radius, double cx, double cy) {
     const int lane = threadIdx.x & 31;
     const int taps = (2 * radius + 1) * (2 * radius + 1);
     const int total = (n + 1) * p.n_targets;
@@ -310,9 +335,11 @@ __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlo
     warp_direct_list<GRID>(p, d, patch, cand, n, n_fast, n_exact);
     __syncwarp();
     const int listed = n_fast + n_exact;
-    for (int j = lane; j < listed; j += 32)
-        direct_item_score<GRID>(p, d, patch, cand, j < n_fast ? d.list[j] : d.list[total - 1 - (j - n_fast)], j < n_fast,
-                          taps);
+    for (int j = lane; j < listed; j += 32) {
+        const int item = j < n_fast ? d.list[j] : d.list[total - 1 - (j - n_fast)], v = item / (n + 1);
+        direct_item_score<GRID, UNROLL>(p, d, patch, cand, n + 1, item, v, direct_taps(p, d, cx, cy, v, radius),
+                                        j < n_fast, taps);
+    }
     __syncwarp();
     warp_direct_aggregate(p, d, n);
 }
@@ -320,7 +347,9 @@ __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlo
 // A warp per fine node; the CTA holds nodes_per_cta nodes. Each warp lists its
 // node's items; the CTA then scores the pooled lists (every node's fast items,
 // then every node's exact items), so the lanes of all warps stay busy up to the
-// pool's last round instead of each node's; each warp then selects its node.
+// pool's last round instead of each node's; each warp then selects its node. It is bound by the
+// L1's data stage (82% of its cycles): items lie target by target, so that neighbouring lanes
+// gather near one another (8.70 -> 8.51 ms at 4160x3120 with four targets).
 // GRID: items on the grid (taps_on_grid) come first and take the f32 form, the others the f64
 // one; without it, the items inside the plane come first and all take the f64 form. The f32
 // form pays where most patches are on the grid, that is away from the plane's left and top
@@ -329,7 +358,7 @@ __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlo
 constexpr int DIRECT_GRID_SIDE = 400;
 
 template <bool GRID>
-__global__ void __launch_bounds__(256) direct_depth_kernel(DirectParams p) {
+__global__ void __launch_bounds__(256, 4) direct_depth_kernel(DirectParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ RefPatch patches[8];
     __shared__ int pool[8][3];  // per node: fast count, exact count, list length
@@ -339,8 +368,9 @@ __global__ void __launch_bounds__(256) direct_depth_kernel(DirectParams p) {
     const bool active = node < p.columns * p.rows;  // whole warps
     const int V = p.n_targets;
     const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
-    const size_t slot_bytes = direct_slot_bytes<float2>(V, taps);
-    DirectSlot<float2> d = carve_direct_slot<float2>(smem_raw + (size_t)slot * slot_bytes, V, taps);
+    const size_t slot_bytes = direct_slot_bytes<float2>(V, taps, MAX_DIRECT_CANDIDATES);
+    DirectSlot<float2> d =
+        carve_direct_slot<float2>(smem_raw + (size_t)slot * slot_bytes, V, taps, MAX_DIRECT_CANDIDATES);
     RefPatch &patch = patches[slot];
     const double cx = (double)((node % p.columns) * p.step), cy = (double)((node / p.columns) * p.step);
     int seeded = 0, n = 0, n_fast = 0, n_exact = 0;
@@ -353,7 +383,7 @@ __global__ void __launch_bounds__(256) direct_depth_kernel(DirectParams p) {
     if (lane == 0) {
         pool[slot][0] = n_fast;
         pool[slot][1] = n_exact;
-        pool[slot][2] = (n + 1) * V;
+        pool[slot][2] = n + 1;
     }
     __syncthreads();
     int fast_total = 0, pooled = 0;
@@ -369,10 +399,13 @@ __global__ void __launch_bounds__(256) direct_depth_kernel(DirectParams p) {
         } else {
             at -= fast_total;
             while (at >= pool[k][1]) at -= pool[k++][1];
-            at = pool[k][2] - 1 - at;
+            at = pool[k][2] * V - 1 - at;
         }
-        const DirectSlot<float2> dk = carve_direct_slot<float2>(smem_raw + (size_t)k * slot_bytes, V, taps);
-        direct_item_score<GRID>(p, dk, patches[k], dk.cand, dk.list[at], j < fast_total, taps);
+        const DirectSlot<float2> dk =
+            carve_direct_slot<float2>(smem_raw + (size_t)k * slot_bytes, V, taps, MAX_DIRECT_CANDIDATES);
+        const int item = dk.list[at], v = item / pool[k][2];
+        direct_item_score<GRID, 3>(p, dk, patches[k], dk.cand, pool[k][2], item, v, direct_taps(p, dk, 0.0, 0.0, v, p.radius),
+                                   j < fast_total, taps);
     }
     __syncthreads();
     if (!active) return;
@@ -402,21 +435,31 @@ __global__ void __launch_bounds__(256) direct_depth_kernel(DirectParams p) {
     }
 }
 
-// The wide-radius retry (depth.rs:803-846) for the listed nodes; a warp per
-// entry, persistent over the list.
-template <bool GRID>
-__global__ void __launch_bounds__(256) direct_wide_kernel(DirectParams p) {
+// The wide-radius retry (depth.rs:803-846) for the listed nodes; a warp per entry, its 8 V
+// correlations lane by lane, persistent over the list: warps take their further entries from a
+// counter, since an entry's work depends on how many of its samples are inside their targets.
+// It waits for samples: what counts is how many warps an SM holds and how much of its memory is
+// left to the L1 cache. A copy of the taps (289 at the default radius, 8 bytes a target) is most
+// of a warp's shared memory, so from three targets on the taps are read from the tap lattice
+// (LATTICE), as lines that neighbouring nodes share. Measured on four targets: 15 warps an SM
+// with the copy and 32 without; direct stage at 4160x3120 14.05 -> 12.68 ms (retry 5.4 -> 4.1),
+// 1567x1173 with three targets 2.05 -> 1.96 ms. With one or two targets the copy fits beside as many
+// warps as the registers allow, and stays: reading the lattice there took 1.84 against 1.75 ms
+// (2080x1560, two targets) and 0.406 against 0.389 ms (1040x780, one).
+template <bool GRID, bool LATTICE>
+__global__ void __launch_bounds__(256, LATTICE ? 0 : 3) direct_wide_kernel(DirectParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ RefPatch patches[8];
     const int slot = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int warps = blockDim.x >> 5;
     const int V = p.n_targets;
     const int taps = (2 * p.wide_radius + 1) * (2 * p.wide_radius + 1);
-    DirectSlot<float2> d =
-        carve_direct_slot<float2>(smem_raw + (size_t)slot * direct_slot_bytes<float2>(V, taps), V, taps);
+    using TapT = typename std::conditional<LATTICE, NoTap, float2>::type;
+    DirectSlot<TapT> d = carve_direct_slot<TapT>(
+        smem_raw + (size_t)slot * direct_slot_bytes<TapT>(V, taps, WIDE_CANDIDATES), V, taps, WIDE_CANDIDATES);
     RefPatch &patch = patches[slot];
     const int count = *p.wide_count;
-    for (int e = blockIdx.x * warps + slot; e < count; e += gridDim.x * warps) {
+    for (int e = blockIdx.x * warps + slot; e < count;) {
         int4 entry = p.wide_list[e];
         const int node = entry.x, first = entry.y, last = entry.z;
         const double cx = (double)((node % p.columns) * p.step), cy = (double)((node / p.columns) * p.step);
@@ -424,7 +467,7 @@ __global__ void __launch_bounds__(256) direct_wide_kernel(DirectParams p) {
         warp_direct_candidates(p, cx, cy, d.cand, seeded);
         warp_stage_node(p, d, patch, cx, cy, p.wide_radius, p.spatial_wide, p.geometry + (size_t)node * V, nullptr);
         const int n = last - first + 1;
-        warp_direct_scores<GRID>(p, d, patch, d.cand + first, n, p.wide_radius);
+        warp_direct_scores<GRID, LATTICE ? 4 : 3>(p, d, patch, d.cand + first, n, p.wide_radius, cx, cy);
         double depth = 0.0;
         float confidence = 0.0f, improvement = 0.0f;
         int best;
@@ -439,6 +482,8 @@ __global__ void __launch_bounds__(256) direct_wide_kernel(DirectParams p) {
             p.out.improvement[node] = improvement;
         }
         __syncwarp();
+        if (lane == 0) e = gridDim.x * warps + atomicAdd(p.wide_count + 1, 1);
+        e = __shfl_sync(0xffffffffu, e, 0);
     }
 }
 

@@ -249,8 +249,8 @@ void set_smem_limits() {
         CK(cudaFuncSetAttribute(cost_kernel_for(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         CK(cudaFuncSetAttribute(cost_node_kernel_for(threads), cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     }
-    for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false>,
-                        direct_wide_kernel<true>})
+    for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false, false>,
+                        direct_wide_kernel<true, false>, direct_wide_kernel<false, true>, direct_wide_kernel<true, true>})
         CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(target_decision_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(target_decision_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -1882,25 +1882,34 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         p.out = direct;
         p.guidance = fguidance;
         p.tested = ftested;
-        p.wide_count = dbuf<int>(ctx, "wide_count", 1);
+        p.wide_count = dbuf<int>(ctx, "wide_count", 2);
         p.wide_list = dbuf<int4>(ctx, "wide_list", M);
-        CK(cudaMemsetAsync(p.wide_count, 0, sizeof(int), s));
+        CK(cudaMemsetAsync(p.wide_count, 0, 2 * sizeof(int), s));
         const int taps = (2 * direct_radius + 1) * (2 * direct_radius + 1);
         const int wide_taps = (2 * wide_radius + 1) * (2 * wide_radius + 1);
-        const size_t slot = direct_slot_bytes<float2>(V, taps), wide_slot = direct_slot_bytes<float2>(V, wide_taps);
-        if (slot > 200 * 1024 || wide_slot > 200 * 1024)
+        const size_t slot = direct_slot_bytes<float2>(V, taps, MAX_DIRECT_CANDIDATES);
+        if (direct_bound_bytes(V, taps) > 200 * 1024 || direct_bound_bytes(V, wide_taps) > 200 * 1024)
             throw CudaError{cudaErrorInvalidValue, "direct pass shared memory exceeds 200 KiB"};
         bool grid = true;  // see DIRECT_GRID_SIDE
         for (int t : targets) grid = grid && std::max(h_views[t].luma.width, h_views[t].luma.height) >= DIRECT_GRID_SIDE;
         const auto direct_kernel = grid ? direct_depth_kernel<true> : direct_depth_kernel<false>;
-        const auto wide_kernel = grid ? direct_wide_kernel<true> : direct_wide_kernel<false>;
         p.nodes_per_cta = warps_per_cta(direct_kernel, slot, 8);
         direct_kernel<<<blocks_for(M, p.nodes_per_cta), 32 * p.nodes_per_cta, p.nodes_per_cta * slot, s>>>(p);
         CK(cudaGetLastError());
-        const int wide_warps = warps_per_cta(wide_kernel, wide_slot, 8);
-        int wide_blocks = 0;
+        // the wide retry copies its taps unless that leaves an SM fewer warps than the registers do
+        auto wide_kernel = grid ? direct_wide_kernel<true, false> : direct_wide_kernel<false, false>;
+        size_t wide_slot = direct_slot_bytes<float2>(V, wide_taps, WIDE_CANDIDATES);
+        int wide_warps = warps_per_cta(wide_kernel, wide_slot, 8), wide_blocks = 0, most_blocks = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_blocks, wide_kernel, 32 * wide_warps,
                                                          wide_warps * wide_slot));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most_blocks, wide_kernel, 256, 0));
+        if (fine_lattice && wide_blocks * wide_warps < most_blocks * 8) {
+            wide_kernel = grid ? direct_wide_kernel<true, true> : direct_wide_kernel<false, true>;
+            wide_slot = direct_slot_bytes<NoTap>(V, wide_taps, WIDE_CANDIDATES);
+            wide_warps = warps_per_cta(wide_kernel, wide_slot, 8);
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_blocks, wide_kernel, 32 * wide_warps,
+                                                             wide_warps * wide_slot));
+        }
         wide_kernel<<<ctx->sm_count * std::max(1, wide_blocks), 32 * wide_warps, wide_warps * wide_slot,
                              s>>>(p);
         CK(cudaGetLastError());

@@ -12,6 +12,8 @@
 // three target sums keep their own sequential order in zncc_score().
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace chiaro {
@@ -67,6 +69,38 @@ __device__ __forceinline__ void store_tap(double2 &d, float qx, float qy) {
     d = make_double2((double)qx * 0.5, (double)qy * 0.5);
 }
 __device__ __forceinline__ void store_tap(float2 &d, float qx, float qy) { d = make_float2(qx * 0.5f, qy * 0.5f); }
+template <typename Half>
+__device__ __forceinline__ float2 tap_half(const Half *taps, int t) {
+    return make_float2((float)taps[t].x, (float)taps[t].y);
+}
+// the coordinates of an f32 tap on the grid: g/2 + offset, rounded once
+__device__ __forceinline__ f32x2 tap_on_grid(const float2 *taps, int t, f32x2 offset) {
+    return add2(pack2(taps[t].x, taps[t].y), offset);
+}
+
+// Taps read where the tap lattice has them, as g: row after row of a patch, `skip` points from
+// the end of one to the start of the next. NoTap stands for them as a slot's tap storage.
+struct NoTap {};
+struct LatticeTaps {
+    const float2 *__restrict__ at;  // the first tap
+    int skip;
+    SmallDiv by_side;
+};
+__device__ __forceinline__ float2 lattice_tap(const LatticeTaps &taps, int t) {
+    return taps.at[t + taps.by_side.quotient(t) * taps.skip];
+}
+__device__ __forceinline__ float2 tap_half(const LatticeTaps &taps, int t) {
+    const float2 g = lattice_tap(taps, t);
+    return make_float2(g.x * 0.5f, g.y * 0.5f);
+}
+__device__ __forceinline__ Tap<float2> load_tap(const LatticeTaps &taps, const float2 *wt, int t) {
+    return {tap_half(taps, t), wt[t]};
+}
+__device__ __forceinline__ f32x2 tap_on_grid(const LatticeTaps &taps, int t, f32x2 offset) {
+    const float2 g = lattice_tap(taps, t);
+    return fma2(pack2(g.x, g.y), pack2(0.5f, 0.5f), offset);  // halving is exact: the same sum
+}
+__device__ __forceinline__ void store_tap(NoTap &, float, float) {}
 
 // The taps of a patch in pairs, for packed arithmetic over both: half = (g/2 x, g/2 x', g/2 y,
 // g/2 y') per target, weight = (w, w', w r, w' r'). A patch has an odd number of taps: the last
@@ -99,14 +133,15 @@ __device__ __forceinline__ TapBox warp_tap_box(const TapBox &b) {
 // eight lanes (min and max are exact, so the reduction order does not matter).
 // Every lane of the warp calls it; the groups reduce with shuffles.
 template <typename TapT>
-__device__ inline TapBox group8_tap_box(const TapT *gh, int taps) {
-    TapBox b{(float)gh[0].x, (float)gh[0].x, (float)gh[0].y, (float)gh[0].y};
+__device__ inline TapBox group8_tap_box(const TapT &gh, int taps) {
+    const float2 first = tap_half(gh, 0);
+    TapBox b{first.x, first.x, first.y, first.y};
     for (int t = threadIdx.x & 7; t < taps; t += 8) {
-        const float gx = (float)gh[t].x, gy = (float)gh[t].y;
-        b.xmin = fminf(b.xmin, gx);
-        b.xmax = fmaxf(b.xmax, gx);
-        b.ymin = fminf(b.ymin, gy);
-        b.ymax = fmaxf(b.ymax, gy);
+        const float2 half = tap_half(gh, t);
+        b.xmin = fminf(b.xmin, half.x);
+        b.xmax = fmaxf(b.xmax, half.x);
+        b.ymin = fminf(b.ymin, half.y);
+        b.ymax = fmaxf(b.ymax, half.y);
     }
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) {
@@ -181,9 +216,17 @@ __global__ void __launch_bounds__(256) tap_lattice_kernel(LatticeParams p) {
     }
 }
 
+// The taps in target v of the patch of the node at (cx, cy), which lies on the lattice.
+__device__ __forceinline__ LatticeTaps lattice_taps(const TapLattice &lattice, double cx, double cy, int v, int radius) {
+    const int side = 2 * radius + 1;
+    return {lattice.planes + (size_t)(v + 1) * lattice.plane_size() + lattice.index(cx, cy) -
+                (ptrdiff_t)radius * (lattice.columns + 1),
+            lattice.columns - side, SmallDiv(side)};
+}
+
 // Warp-cooperative staging of one node at (cx, cy) and `radius`: the
 // reference patch ((w, w r) and (w r) r per tap, the three sums, the energy and the
-// centre sample) and, for each target, g/2 of every tap and their box. Returns
+// centre sample) and, for each target, every tap (store_tap) and the box of their g/2. Returns
 // on every lane the mask of targets with a tap where the global warp is None
 // (bit v); `patch` is written by lanes 0-2 and valid after the trailing
 // __syncwarp(). `pre`: the node's patch from patch_sums_kernel at this radius, or
@@ -242,7 +285,12 @@ __device__ inline unsigned warp_stage_patch(const DevView *views, int reference,
     __syncwarp();
     for (int vb = 0; vb < V; vb += 4) {  // eight lanes per target
         const int v = vb + (lane >> 3);
-        TapBox b = group8_tap_box(gh + (v < V ? v : V - 1) * taps, taps);
+        const int vs = v < V ? v : V - 1;
+        TapBox b;
+        if constexpr (std::is_same<TapT, NoTap>::value)
+            b = group8_tap_box(lattice_taps(lattice, cx, cy, vs, radius), taps);
+        else
+            b = group8_tap_box(static_cast<const TapT *>(gh + vs * taps), taps);
         if ((lane & 7) == 0 && v < V) box[v] = b;
     }
     if (pre) {
@@ -630,14 +678,14 @@ __device__ __forceinline__ float zncc_grid(const float4 *__restrict__ quads, int
     float st = 0.0f, stt = 0.0f, srt = 0.0f;
 #pragma unroll UNROLL
     for (int t = 0; t < taps; ++t) {
-        const auto tap = load_tap(gh, wt, t);
-        const f32x2 x = add2(pack2(tap.half.x, tap.half.y), e);
+        const float2 weights = wt[t];
+        const f32x2 x = tap_on_grid(gh, t, e);
         const f32x2 m = add2_down(x, magic);
         const f32x2 frac = fma2(add2(m, minus_magic), minus_one, x), rest = fma2(frac, minus_one, one);
         const float2 mf = unpack2(m);
         const int ix = (int)(f2u(mf.x) - 0x4B000000u), iy = (int)(f2u(mf.y) - 0x4B000000u);
         const float4 q = __ldg(quads + quad_index(ix, iy, stride));
-        add_sample(q, unpack2(frac), unpack2(rest), tap.weights, st, stt, srt);
+        add_sample(q, unpack2(frac), unpack2(rest), weights, st, stt, srt);
     }
     return zncc_finish(patch, st, stt, srt, ok);
 }
