@@ -38,7 +38,8 @@ struct DecisionParams {
     Decisions out[MAX_VIEWS];  // per target (index into targets)
 };
 
-constexpr int decision_warps(bool pooled) { return pooled ? 8 : 4; }  // most nodes (warps) per CTA
+constexpr int DECISION_WARPS = 4;   // most nodes (warps) per CTA
+constexpr int DECISION_UNROLL = 4;  // taps in flight a lane
 
 // Per-warp shared memory of the decisions for V targets and T taps.
 struct DecisionSlot {
@@ -107,11 +108,10 @@ __device__ __forceinline__ int list_items(const DecisionSlot &d, int count, bool
 
 // The correlation of d's listed entry `at` (target v). The f64 form alone (zncc_any): a node
 // lists 24 or 32 items for one warp, so one item off the grid would cost the warp both loops.
-template <int UNROLL>
 __device__ __forceinline__ bool decision_score(const DecisionParams &p, const DecisionSlot &d, const RefPatch &patch,
                                                int at, int v, int taps, float &score) {
     const double2 dd = d.disp[at];
-    return zncc_any<UNROLL>(p.views[p.targets[v]], d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y, score);
+    return zncc_any<DECISION_UNROLL>(p.views[p.targets[v]], d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y, score);
 }
 
 // Scores the pooled lists of the CTA's nodes (node k's count[k] entries of its
@@ -132,7 +132,7 @@ __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned ch
         const int item = d.list[at];
         const int v = shifts ? item >> 3 : item / 6;
         float score;
-        const bool ok = decision_score<9>(p, d, patches[k], at, v, taps, score);
+        const bool ok = decision_score(p, d, patches[k], at, v, taps, score);
         const int kk = shifts ? 6 + (item & 7) : item - v * 6;
         if (ok)
             d.sc[v * 16 + kk] = score;
@@ -148,17 +148,18 @@ __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned ch
 // node): the CTA scores the pooled lists of all its nodes instead, so few warps
 // issue each phase's correlations; nodes without work stay for the CTA's
 // barriers.
-// The kernel waits for samples, so it wants warps: without pooling a warp is on its own, and CTAs
-// of four with 64 registers give an SM 32 of them (24 of 75 registers in CTAs of eight, where a
-// node without a depth also keeps its slot until the CTA's other nodes are done). That leaves
-// room for four taps in flight a lane instead of nine. Measured, decisions: 4160x3120 with four
-// targets 5.28 -> 4.72 ms, 3120x2340 with three 2.19 -> 1.93, 1567x1173 with three 0.517 -> 0.501;
-// CTAs of two 4.67 / 1.98 / 0.517, of one 4.88 / 2.02 / 0.526; 48 registers 5.69 ms.
+// The kernel waits for samples, so it wants warps: CTAs of four nodes with 64 registers give an SM
+// 32 of them (24 of 75 registers in CTAs of eight, whose barriers, or slots kept until the CTA is
+// done, also cost more). That leaves room for four taps in flight a lane instead of nine.
+// Measured, decisions: 4160x3120 with four targets 5.28 -> 4.72 ms, 3120x2340 with three 2.19 ->
+// 1.93, 1567x1173 with three 0.517 -> 0.501; pooled, 2080x1560 with two 1.021 -> 0.865, 1040x780
+// with one 0.378 -> 0.349. Without pooling, CTAs of two 4.67 / 1.98 / 0.517, of one 4.88 / 2.02 /
+// 0.526; 48 registers 5.69 ms.
 template <bool POOLED>
-__global__ void __launch_bounds__(32 * decision_warps(POOLED), POOLED ? 0 : 32 / decision_warps(false)) target_decision_kernel(DecisionParams p) {
+__global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) target_decision_kernel(DecisionParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ RefPatch patches[decision_warps(POOLED)];
-    __shared__ int count[decision_warps(POOLED)];
+    __shared__ RefPatch patches[DECISION_WARPS];
+    __shared__ int count[DECISION_WARPS];
     const unsigned full = 0xffffffffu;
     const int slot = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nodes = blockDim.x >> 5;
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(32 * decision_warps(POOLED), POOLED ? 0 : 32 /
             const int item = d.list[j];
             const int v = item / 6, k = item - v * 6;
             float score;
-            if (decision_score<4>(p, d, patch, j, v, taps, score))
+            if (decision_score(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + k] = score;
             else if (k < 5)
                 atomicOr(&d.flags[v], 1);
@@ -304,7 +305,7 @@ __global__ void __launch_bounds__(32 * decision_warps(POOLED), POOLED ? 0 : 32 /
             const int item = d.list[j];
             const int v = item >> 3;
             float score;
-            if (decision_score<4>(p, d, patch, j, v, taps, score))
+            if (decision_score(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + 6 + (item & 7)] = score;
             else
                 atomicOr(&d.flags[v], 1);

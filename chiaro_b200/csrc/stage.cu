@@ -2005,7 +2005,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         // one or two targets leave most lanes of a node's warp idle in both phases (6 V and
         // 8 V items): the CTA then pools its nodes' correlations
         const auto decision_kernel = V <= 2 ? target_decision_kernel<true> : target_decision_kernel<false>;
-        const int warps = warps_per_cta(decision_kernel, slot, decision_warps(V <= 2));
+        const int warps = warps_per_cta(decision_kernel, slot, DECISION_WARPS);
         decision_kernel<<<blocks_for(M, warps), 32 * warps, warps * slot, s>>>(p);
         CK(cudaGetLastError());
         WarpPasses w{};
