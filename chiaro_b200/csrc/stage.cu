@@ -69,8 +69,8 @@ struct chiaro_depth_ctx {
     int union_retries = -1;
     uint64_t memory_limit = 0;
     uint64_t memory_held = 0;
-    // launch shapes chosen by the autotuner: cost-volume threads per node CTA per bucket;
-    // autotune: 1 tune, 0 the default shape, or a forced shape (threads per node CTA)
+    // launch shapes chosen by the autotuner: cost-volume threads per CTA per bucket and form
+    // (launch_cost); autotune: 1 tune, 0 the default shape, or a forced shape (threads per CTA)
     int autotune = 1;
     std::map<uint64_t, int> cost_tuning;
 };
@@ -319,10 +319,13 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
 }
 
 // Launch build_cost_volume over n_rows nodes. With autotuning on, the first launch of a
-// (targets, labels scored, radius) bucket large enough to time (at least 4096 nodes, outside
-// any stream capture) runs every shape twice and keeps the fastest second run for the
-// context's later launches; every shape writes the same bits, and the last launch below
-// writes the outputs again.
+// (targets, labels scored, radius) bucket in a form of the kernel (node by node, or in tiles of
+// so many nodes, targets in turn or side by side) large enough to time (at least 4096 nodes,
+// outside any stream capture) runs every shape twice and keeps the fastest second run for the
+// context's later launches of that bucket and form: the forms' CTAs do different work, so one's
+// choice says nothing about another's. Every shape writes the same bits, and the last launch
+// below writes the outputs again.
+constexpr uint64_t COST_BUCKET_MASK = ((uint64_t)1 << 40) - 1;  // of a key: its bucket; the form lies above
 void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView> &views, size_t n_rows,
                  size_t path_floats) {
     cudaStream_t s = ctx->stream;
@@ -351,7 +354,9 @@ void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView>
             cost_node_kernel_for(threads)<<<blocks, threads, smem, s>>>(p);
         CK(cudaGetLastError());
     };
-    const uint64_t key = ((uint64_t)p.n_targets << 24) | ((uint64_t)p.slots << 8) | (uint64_t)p.radius;
+    const uint64_t form = tiles ? (uint64_t)(p.tile_w * p.tile_h) << 1 | (turns > 1 ? 1 : 0) : 0;
+    const uint64_t key =
+        form << 40 | (uint64_t)p.n_targets << 24 | (uint64_t)p.slots << 8 | (uint64_t)p.radius;
     int threads = ctx->autotune > 1 ? ctx->autotune : COST_THREADS;
     auto it = ctx->cost_tuning.find(key);
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
@@ -2381,7 +2386,7 @@ int chiaro_depth_tuning(const chiaro_depth_ctx *ctx, uint64_t *keys, int32_t *th
     int n = 0;
     for (const auto &kv : ctx->cost_tuning) {
         if (n < capacity) {
-            if (keys) keys[n] = kv.first;
+            if (keys) keys[n] = kv.first & COST_BUCKET_MASK;
             if (threads) threads[n] = kv.second;
         }
         ++n;

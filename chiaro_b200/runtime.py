@@ -232,7 +232,8 @@ class DepthContext:
         self.check(self.lib.chiaro_depth_set_autotune(self.handle, int(mode)))
 
     def tuning(self) -> dict:
-        """The autotuner's choices: {(targets, labels scored, radius): threads per node CTA}."""
+        """The autotuner's choices: {(targets, labels scored, radius): threads per CTA}; of a bucket
+        that ran in several forms of the cost volume, the one for the largest tiles."""
         n = int(self.lib.chiaro_depth_tuning(self.handle, None, None, 0))
         keys = (C.c_uint64 * max(n, 1))()
         threads = (C.c_int32 * max(n, 1))()

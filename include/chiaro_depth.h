@@ -292,12 +292,13 @@ uint64_t chiaro_depth_memory_held(const chiaro_depth_ctx *ctx);
 /* No counterpart in the reference: launch-shape autotuning. With mode 1 (the default),
  * the first cost-volume launch of each (targets, labels scored, patch radius) bucket with
  * at least 4096 nodes, outside any stream capture, times every candidate CTA size (64, 96,
- * 128, 160 and 192 threads per node) and keeps the fastest for the context's later launches.
- * Every size gives the same bits. Mode 0 runs the default of 128 threads; mode 64, 96, 128,
+ * 128, 160 and 192 threads) and keeps the fastest for the context's later launches. The
+ * cost volume has several forms, taken by the sizes of the planes and the grid; a bucket is
+ * timed in each form that it runs in. Every size gives the same bits. Mode 0 runs the default of 128 threads; mode 64, 96, 128,
  * 160 or 192 runs that size everywhere; both forget the choices made. Other modes return
  * CHIARO_ERR_ARGUMENT. chiaro_depth_tuning writes up to `capacity` choices, each a bucket
  * key ((targets << 24) | (labels scored << 8) | radius) and its threads, and returns how
- * many the context holds. */
+ * many the context holds; a bucket that ran in several forms has a choice for each. */
 int chiaro_depth_set_autotune(chiaro_depth_ctx *ctx, int32_t mode);
 int chiaro_depth_tuning(const chiaro_depth_ctx *ctx, uint64_t *keys, int32_t *threads, int capacity);
 

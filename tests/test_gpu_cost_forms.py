@@ -1,0 +1,46 @@
+"""The cost volume's forms side by side (GPU): node by node on small planes and grids, in node
+tiles on the others, with the targets in turn or side by side (launch_cost). Each is tuned by
+itself."""
+import pytest
+
+from chiaro_b200 import scenes
+from chiaro_b200.depth import DepthOptions, refine_multiview_depth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture()
+def ctx():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from chiaro_b200.runtime import DepthContext
+    c = DepthContext(0)
+    yield c
+    c.close()
+
+
+def make_case(width, height, sources, planes, seed=3, step=8, radius=4, focal=None, support=None):
+    support = support or (1 if sources == 1 else 2)
+    opt = DepthOptions(grid_step=step, planes=planes, patch_radius=radius, near_depth=400.0, far_depth=25000.0,
+                       minimum_support=support, best_view_count=max(support, 3))
+    return scenes.make_scene("forms", width, height, sources, 5, 1, (500.0, 8000.0), (20.0, 60.0), 0.4, opt, seed,
+                             distortion=True, focal_px=focal)
+
+
+def run(ctx, scene, debug=None):
+    alignments = scene.alignments()
+    dmap = refine_multiview_depth(scene.inputs(), 0, alignments, scene.options, context=ctx, debug=debug)
+    assert dmap is not None
+    return dmap, alignments
+
+
+# (both of at least 4096 nodes, with one target and 65 labels)
+@pytest.mark.parametrize("order", [(0, 1), (1, 0)])
+def test_the_forms_of_a_bucket_are_tuned_apart(ctx, order):
+    rasters = [(723, 531), (1000, 700)]  # below and above the 600,000 hypotheses from which tiles pay
+    for n, i in enumerate(order):
+        width, height = rasters[i]
+        run(ctx, make_case(width, height, 1, 64))
+        assert int(ctx.lib.chiaro_depth_tuning(ctx.handle, None, None, 0)) == n + 1
+        assert list(ctx.tuning()) == [(1, 65, 4)]  # the reported key is the bucket's
