@@ -219,11 +219,50 @@ CostNodeKernel cost_node_kernel_for(int threads) {
 // target and 65 labels, 0.41 M items: 81 -> 65 us and 15 us of set-up; 1040x780, 0.84 M: 310 -> 240).
 constexpr size_t COST_TILE_ITEMS = 600000;
 
-bool cost_in_tiles(const std::vector<DevView> &views, const std::vector<int> &targets, size_t nodes, int labels) {
+// The extent in samples of a target's epipolar segment from infinity to `near_depth`, at the
+// reference's centre. Where the near end lies outside the target's frame (more than half its
+// size, which projects to nothing), the part as far as a multiple of that depth is measured and
+// scaled: a displacement from infinity goes with the inverse depth. False where there is none.
+bool epipolar_extent(const DevView &rv, const DevView &tv, double near_depth, double &dx, double &dy) {
+    D3 origin, direction;
+    double x0, y0, x1, y1;
+    pixel_to_ray(rv.cam, rv.width * 0.5, rv.height * 0.5, origin, direction);
+    if (!project(tv.cam, along(origin, direction, INFINITY_DEPTH), x0, y0)) return false;
+    for (double scale = 1.0; near_depth * scale < INFINITY_DEPTH; scale *= 2.0)
+        if (project(tv.cam, along(origin, direction, near_depth * scale), x1, y1)) {
+            dx = std::fabs(x1 - x0) * 0.5 * scale;
+            dy = std::fabs(y1 - y0) * 0.5 * scale;
+            return std::isfinite(dx) && std::isfinite(dy);
+        }
+    return false;
+}
+
+// Segments far longer than a hypothesis's reach (64 samples either way) leave most labels out of
+// it: a tile's part of the labels then holds few scored items, or none, and pays its listing,
+// copy and barriers all the same, while a node's CTA lists every target's few items together.
+// So the targets' segments, summed, are bounded: more on a grid large enough to hide a part's
+// barriers behind other CTAs, and more again where there are at most three targets to list.
+// Node / tile in ms, by that sum. 12,838 nodes (1040x780): three targets, 129 labels, 834: 0.44 /
+// 0.40; two, 129, 1096: 0.28 / 0.28; four, 65, 1182: 0.36 / 0.44. 26,790 nodes (1500x1125), 97
+// labels: three targets, 998: 0.67 / 0.60; two, 1024: 0.45 / 0.49; four, 1418: 0.80 / 0.86. 51,000
+// nodes (2080x1560): four targets, 65 labels, 1176: 1.27 / 1.18, 1568: 1.12 / 1.19; five, 129,
+// 1350: 2.51 / 2.46, 2725: 1.87 / 2.36; three, 129, 1665: 1.16 / 1.12, 2238: 1.13 / 1.33.
+// 203,711 nodes (4160x3120), 97 labels: four targets, 1249: 6.05 / 5.73, 2347: 4.80 / 5.93; three,
+// 1649: 4.14 / 3.72.
+constexpr size_t COST_TILE_LARGE_GRID = 40000;
+constexpr double COST_TILE_SEGMENTS[] = {1000.0, 1300.0, 2000.0};  // small grid; large; large, at most three targets
+
+bool cost_in_tiles(const std::vector<DevView> &views, int reference, const std::vector<int> &targets, double near_depth,
+                   size_t nodes, int labels) {
     if (nodes * targets.size() * labels < COST_TILE_ITEMS) return false;
     int side = 0;
-    for (int t : targets) side = std::max({side, views[t].luma.width, views[t].luma.height});
-    return side >= COST_TILE_SIDE;
+    double segments = 0.0, dx, dy;
+    for (int t : targets) {
+        side = std::max({side, views[t].luma.width, views[t].luma.height});
+        if (epipolar_extent(views[reference], views[t], near_depth, dx, dy)) segments += std::max(dx, dy);
+    }
+    const int grid = nodes < COST_TILE_LARGE_GRID ? 0 : targets.size() > 3 ? 1 : 2;
+    return side >= COST_TILE_SIDE && segments <= COST_TILE_SEGMENTS[grid];
 }
 
 CostKernel cost_kernel_for(int threads) {
@@ -292,14 +331,8 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
         const DevView &tv = views[p.targets[v]];
         p.transposed[v] = 0;
         p.passes[v] = 1;
-        D3 origin, direction;
-        double x0, y0, x1, y1;
-        pixel_to_ray(rv.cam, rv.width * 0.5, rv.height * 0.5, origin, direction);
-        if (!project(tv.cam, along(origin, direction, INFINITY_DEPTH), x0, y0) ||
-            !project(tv.cam, along(origin, direction, p.near_depth), x1, y1))
-            continue;
-        const double dx = std::fabs(x1 - x0) * 0.5, dy = std::fabs(y1 - y0) * 0.5;  // samples
-        if (!(std::isfinite(dx) && std::isfinite(dy))) continue;
+        double dx, dy;
+        if (!epipolar_extent(rv, tv, p.near_depth, dx, dy)) continue;
         p.transposed[v] = dy > dx;
         // the share of the segment that the scored labels cover, and the room for it beside the
         // patch, the tile's nodes, the bilinear neighbour, alignment and the warp's own bending
@@ -1311,7 +1344,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     launch_sample_planes(ctx, g.views, h_views, g.targets);
     g.h_views = h_views;
     const auto full_range_patches = [&] {  // the node tiles of a full-range cost volume read them
-        if (!cost_in_tiles(h_views, g.targets, N, D)) return;
+        if (!cost_in_tiles(h_views, reference, g.targets, o.near_depth, N, D)) return;
         g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
         launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
     };
@@ -1760,7 +1793,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     RefPatch *coarse_patches = nullptr;  // the node tiles of the cost volume read them
     std::vector<PatchGrid> patch_grids{{(int)g.columns, (int)g.rows, (int)g.step, direct_radius, d_sp_direct,
                                         fine_lattice ? lattice : TapLattice{}, fine_patches}};
-    if (cost_in_tiles(h_views, targets, N, D)) {
+    if (cost_in_tiles(h_views, reference, targets, o.near_depth, N, D)) {
         coarse_patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
         patch_grids.push_back({(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, radius, d_sp,
                                coarse_lattice ? lattice : TapLattice{}, coarse_patches});

@@ -44,3 +44,22 @@ def test_the_forms_of_a_bucket_are_tuned_apart(ctx, order):
         run(ctx, make_case(width, height, 1, 64))
         assert int(ctx.lib.chiaro_depth_tuning(ctx.handle, None, None, 0)) == n + 1
         assert list(ctx.tuning()) == [(1, 65, 4)]  # the reported key is the bucket's
+
+
+# The segments' sum in samples is some 470 and 6200 here.
+def test_segments_far_beyond_the_reach_go_node_by_node(ctx):
+    """Two lenses, one bucket and raster: the long lens spreads the labels far beyond a
+    hypothesis's reach and takes the other form, which is timed by itself. Both are the oracle's."""
+    import numpy as np
+    from chiaro_b200.depth import output_shape
+    from oracle import oracle
+    for n, focal in enumerate((2500.0, 15000.0)):
+        scene = make_case(700, 520, 4, 96, focal=focal)
+        (columns, rows, _), (cc, cr, _) = output_shape(scene.width, scene.height, scene.options)
+        buffers = [oracle.debug_buffers(5, cc * cr, 97, columns * rows) for _ in range(2)]
+        run(ctx, scene, buffers[0])
+        assert int(ctx.lib.chiaro_depth_tuning(ctx.handle, None, None, 0)) == n + 1
+        oracle.refine_multiview_depth(scene.inputs(), 0, scene.alignments(), scene.options, threads=8, debug=buffers[1])
+        assert buffers[1]["coarse_tested"].any()
+        for key in ("coarse_scores", "coarse_costs", "coarse_guidance", "coarse_tested"):
+            assert np.array_equal(buffers[0][key].view(np.uint8), buffers[1][key].view(np.uint8)), key
