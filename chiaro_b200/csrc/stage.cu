@@ -1929,7 +1929,10 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         if (direct_bound_bytes(V, taps) > 200 * 1024 || direct_bound_bytes(V, wide_taps) > 200 * 1024)
             throw CudaError{cudaErrorInvalidValue, "direct pass shared memory exceeds 200 KiB"};
         bool grid = true;  // see DIRECT_GRID_SIDE
-        for (int t : targets) grid = grid && std::max(h_views[t].luma.width, h_views[t].luma.height) >= DIRECT_GRID_SIDE;
+        for (int t : targets) {
+            const int side = std::max(h_views[t].luma.width, h_views[t].luma.height);
+            grid = grid && side >= DIRECT_GRID_SIDE && side <= GRID_OFFSET_MAX_SIDE;
+        }
         const auto direct_kernel = grid ? direct_depth_kernel<true> : direct_depth_kernel<false>;
         p.nodes_per_cta = warps_per_cta(direct_kernel, slot, 8);
         direct_kernel<<<blocks_for(M, p.nodes_per_cta), 32 * p.nodes_per_cta, p.nodes_per_cta * slot, s>>>(p);

@@ -1,10 +1,11 @@
 """The cost volume's forms side by side (GPU): node by node on small planes and grids, in node
 tiles on the others, with the targets in turn or side by side (launch_cost). Each is tuned by
 itself."""
+import numpy as np
 import pytest
 
 from chiaro_b200 import scenes
-from chiaro_b200.depth import DepthOptions, refine_multiview_depth
+from chiaro_b200.depth import DepthOptions, output_shape, refine_multiview_depth
 
 pytestmark = pytest.mark.gpu
 
@@ -35,6 +36,26 @@ def run(ctx, scene, debug=None):
     return dmap, alignments
 
 
+def compare_with_the_oracle(ctx, scene, direct=False):
+    """Runs the stage and compares its cost volume (and its direct pass) with the oracle's, bit
+    for bit; returns the oracle's flags of the nodes that scored."""
+    from oracle import oracle
+    (columns, rows, _), (cc, cr, _) = output_shape(scene.width, scene.height, scene.options)
+    views = len(scene.cameras)
+    got, expected = (oracle.debug_buffers(views, cc * cr, scene.options.planes + 1, columns * rows) for _ in range(2))
+    run(ctx, scene, got)
+    oracle.refine_multiview_depth(scene.inputs(), 0, scene.alignments(), scene.options, threads=8, debug=expected)
+    keys = ["coarse_scores", "coarse_costs", "coarse_guidance", "coarse_tested"]
+    if direct:
+        keys += ["direct_has", "direct_tested", "direct_guidance"]
+        has = expected["direct_has"] == 1
+        for key in ("direct_depth", "direct_confidence", "direct_improvement"):
+            assert np.array_equal(got[key][has].view(np.uint8), expected[key][has].view(np.uint8)), key
+    for key in keys:
+        assert np.array_equal(got[key].view(np.uint8), expected[key].view(np.uint8)), key
+    return expected["coarse_tested"]
+
+
 # (both of at least 4096 nodes, with one target and 65 labels)
 @pytest.mark.parametrize("order", [(0, 1), (1, 0)])
 def test_the_forms_of_a_bucket_are_tuned_apart(ctx, order):
@@ -50,16 +71,14 @@ def test_the_forms_of_a_bucket_are_tuned_apart(ctx, order):
 def test_segments_far_beyond_the_reach_go_node_by_node(ctx):
     """Two lenses, one bucket and raster: the long lens spreads the labels far beyond a
     hypothesis's reach and takes the other form, which is timed by itself. Both are the oracle's."""
-    import numpy as np
-    from chiaro_b200.depth import output_shape
-    from oracle import oracle
     for n, focal in enumerate((2500.0, 15000.0)):
         scene = make_case(700, 520, 4, 96, focal=focal)
-        (columns, rows, _), (cc, cr, _) = output_shape(scene.width, scene.height, scene.options)
-        buffers = [oracle.debug_buffers(5, cc * cr, 97, columns * rows) for _ in range(2)]
-        run(ctx, scene, buffers[0])
+        assert compare_with_the_oracle(ctx, scene).any()
         assert int(ctx.lib.chiaro_depth_tuning(ctx.handle, None, None, 0)) == n + 1
-        oracle.refine_multiview_depth(scene.inputs(), 0, scene.alignments(), scene.options, threads=8, debug=buffers[1])
-        assert buffers[1]["coarse_tested"].any()
-        for key in ("coarse_scores", "coarse_costs", "coarse_guidance", "coarse_tested"):
-            assert np.array_equal(buffers[0][key].view(np.uint8), buffers[1][key].view(np.uint8)), key
+
+
+# The luminance side at which no sample position is taken in f32 any more is 8192.
+@pytest.mark.parametrize("width,sources", [(16384, 1), (16400, 3)])
+def test_planes_beyond_the_f32_positions(ctx, width, sources):
+    scene = make_case(width, 150, sources, 16, radius=3, focal=3000.0)
+    assert compare_with_the_oracle(ctx, scene, direct=True).any()
