@@ -632,8 +632,10 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_node_kernel(CostParam
         if (fast)
             score = zncc_inside<9>(tv.quads, tv.quad_stride, s.gh + v * taps, s.wt, patch, taps, dd.x * 0.5, dd.y * 0.5,
                                    ok);
-        else
-            ok = zncc_score(tv.luma, s.gh + v * taps, s.wt, patch, taps, dd.x, dd.y, score);
+        else {
+            const PlaneRef plane = tv.luma;  // in registers over the taps (see zncc_any)
+            ok = zncc_score(plane, s.gh + v * taps, s.wt, patch, taps, dd.x, dd.y, score);
+        }
         s.score[item] = ok ? score : NAN;
     }
     __syncthreads();
