@@ -228,13 +228,25 @@ __device__ inline void warp_stage_node(const DirectParams &p, const DirectSlot<T
     __syncwarp();
 }
 
+// The items of a node: candidate c in [-1, n) (-1 is the baseline) in target v. By target,
+// neighbouring lanes sample one target, near one another; by candidate, neighbouring lanes hold
+// one candidate's targets.
+template <bool BY_TARGET>
+struct DirectItems {
+    int count, V;  // candidates with the baseline, targets
+    __device__ __forceinline__ int item(int v, int c) const { return BY_TARGET ? v * count + c + 1 : (c + 1) * V + v; }
+    __device__ __forceinline__ int target(int item) const { return BY_TARGET ? item / count : item % V; }
+    __device__ __forceinline__ int candidate(int item, int v) const {
+        return (BY_TARGET ? item - v * count : item / V) - 1;
+    }
+};
+
 // Warp-cooperative listing of the baseline and candidates cand[0..n) over all
-// targets. Item v (n + 1) + c + 1 is candidate c in target v, candidate -1 being the
-// baseline: neighbouring lanes sample one target. It settles which items reach the correlation and which of them are fast (on
+// targets (DirectItems). It settles which items reach the correlation and which of them are fast (on
 // the grid, their offset in d.items; without GRID, inside the plane), sets the others'
 // scores to None and lists the scored ones: fast from the front of d.list, the rest from the
 // back of its (n + 1) V entries. Every lane returns the two counts.
-template <bool GRID, typename TapT>
+template <bool GRID, bool BY_TARGET, typename TapT>
 __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<TapT> &d, const RefPatch &patch,
                                         const double *cand, int n, int &n_fast, int &n_exact) {
     const unsigned full = 0xffffffffu;
@@ -242,7 +254,7 @@ __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<
     const unsigned below = (1u << lane) - 1u;
     const int V = p.n_targets;
     const int total = (n + 1) * V;
-    const SmallDiv by_target(n + 1);
+    const SmallDiv split(BY_TARGET ? n + 1 : V);
     const ViewGeom *geom = d.geom;
     n_fast = 0;
     n_exact = 0;
@@ -250,7 +262,8 @@ __device__ inline void warp_direct_list(const DirectParams &p, const DirectSlot<
         const int item = base + lane;
         bool scored = false, fast = false;
         if (item < total) {
-            const int v = by_target.quotient(item), c = item - v * (n + 1) - 1;
+            const int quotient = split.quotient(item), rest = item - quotient * (int)split.d;
+            const int v = BY_TARGET ? quotient : rest, c = (BY_TARGET ? rest : quotient) - 1;
             const ViewGeom &g = geom[v];
             double ddx = 0.0, ddy = 0.0;
             bool ok = g.gc_ok;
@@ -288,13 +301,12 @@ __device__ __forceinline__ auto direct_taps(const DirectParams &p, const DirectS
         return static_cast<const TapT *>(d.gh + v * (2 * radius + 1) * (2 * radius + 1));
 }
 
-// The correlation of one listed item (warp_direct_list) of `count` a target into d.items, with
-// its target's taps; one thread. `fast`: listed as on the grid.
+// The correlation of candidate c in target v, listed as `item` (warp_direct_list), into d.items,
+// with its target's taps; one thread. `fast`: listed as on the grid.
 template <bool GRID, int UNROLL, typename TapT, typename Taps>
 __device__ __forceinline__ void direct_item_score(const DirectParams &p, const DirectSlot<TapT> &d,
-                                                  const RefPatch &patch, const double *cand, int count, int item,
-                                                  int v, const Taps &tap, bool fast, int taps) {
-    const int c = item - v * count - 1;
+                                                  const RefPatch &patch, const double *cand, int item, int v, int c,
+                                                  const Taps &tap, bool fast, int taps) {
     const DevView &tv = p.views[p.targets[v]];
     float score;
     bool ok;
@@ -310,12 +322,13 @@ __device__ __forceinline__ void direct_item_score(const DirectParams &p, const D
 
 // aggregate (depth.rs:1761-1770) of the baseline and candidates over the targets into
 // d.agg[0..n]; the warp of the node.
-template <typename TapT>
+template <bool BY_TARGET, typename TapT>
 __device__ inline void warp_direct_aggregate(const DirectParams &p, const DirectSlot<TapT> &d, int n) {
     const int V = p.n_targets;
+    const DirectItems<BY_TARGET> items{n + 1, V};
     for (int c = threadIdx.x & 31; c <= n; c += 32) {
         float sc[MAX_VIEWS];
-        for (int v = 0; v < V; ++v) sc[v] = d.items[v * (n + 1) + c].x;
+        for (int v = 0; v < V; ++v) sc[v] = d.items[items.item(v, c - 1)].x;
         float a;
         d.agg[c] = aggregate_scores(sc, V, p.minimum_support, p.best_view_count, a) ? a : NAN;
     }
@@ -332,24 +345,28 @@ __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlo
     const int taps = (2 * radius + 1) * (2 * radius + 1);
     const int total = (n + 1) * p.n_targets;
     int n_fast, n_exact;
-    warp_direct_list<GRID>(p, d, patch, cand, n, n_fast, n_exact);
+    warp_direct_list<GRID, true>(p, d, patch, cand, n, n_fast, n_exact);
     __syncwarp();
+    const DirectItems<true> items{n + 1, p.n_targets};
     const int listed = n_fast + n_exact;
     for (int j = lane; j < listed; j += 32) {
-        const int item = j < n_fast ? d.list[j] : d.list[total - 1 - (j - n_fast)], v = item / (n + 1);
-        direct_item_score<GRID, UNROLL>(p, d, patch, cand, n + 1, item, v, direct_taps(p, d, cx, cy, v, radius),
-                                        j < n_fast, taps);
+        const int item = j < n_fast ? d.list[j] : d.list[total - 1 - (j - n_fast)], v = items.target(item);
+        direct_item_score<GRID, UNROLL>(p, d, patch, cand, item, v, items.candidate(item, v),
+                                        direct_taps(p, d, cx, cy, v, radius), j < n_fast, taps);
     }
     __syncwarp();
-    warp_direct_aggregate(p, d, n);
+    warp_direct_aggregate<true>(p, d, n);
 }
 
 // A warp per fine node; the CTA holds nodes_per_cta nodes. Each warp lists its
 // node's items; the CTA then scores the pooled lists (every node's fast items,
 // then every node's exact items), so the lanes of all warps stay busy up to the
 // pool's last round instead of each node's; each warp then selects its node. It is bound by the
-// L1's data stage (82% of its cycles): items lie target by target, so that neighbouring lanes
-// gather near one another (8.70 -> 8.51 ms at 4160x3120 with four targets).
+// L1's data stage (82% of its cycles): with GRID items lie target by target, so that neighbouring
+// lanes gather near one another (8.70 -> 8.51 ms at 4160x3120 with four targets). Without, on
+// planes small enough to lie in the L1, there is nothing to gain by that, and a target whose
+// patches cross an edge fills whole warps with the slower exact path: by candidate there (400x300,
+// four targets: 0.60 -> 0.54 ms at radius 8, 0.174 -> 0.157 at radius 4).
 // GRID: items on the grid (taps_on_grid) come first and take the f32 form, the others the f64
 // one; without it, the items inside the plane come first and all take the f64 form. The f32
 // form pays where most patches are on the grid, that is away from the plane's left and top
@@ -380,7 +397,7 @@ __global__ void __launch_bounds__(256, 4) direct_depth_kernel(DirectParams p) {
         n = warp_direct_candidates(p, cx, cy, d.cand, seeded);
         warp_stage_node(p, d, patch, cx, cy, p.radius, p.spatial, p.geometry + (size_t)node * V,
                         p.patches ? p.patches + node : nullptr);
-        warp_direct_list<GRID>(p, d, patch, d.cand, n, n_fast, n_exact);
+        warp_direct_list<GRID, GRID>(p, d, patch, d.cand, n, n_fast, n_exact);
     }
     if (lane == 0) {
         pool[slot][0] = n_fast;
@@ -405,13 +422,14 @@ __global__ void __launch_bounds__(256, 4) direct_depth_kernel(DirectParams p) {
         }
         const DirectSlot<float2> dk =
             carve_direct_slot<float2>(smem_raw + (size_t)k * slot_bytes, V, taps, MAX_DIRECT_CANDIDATES);
-        const int item = dk.list[at], v = item / pool[k][2];
-        direct_item_score<GRID, 3>(p, dk, patches[k], dk.cand, pool[k][2], item, v, direct_taps(p, dk, 0.0, 0.0, v, p.radius),
-                                   j < fast_total, taps);
+        const DirectItems<GRID> items{pool[k][2], V};
+        const int item = dk.list[at], v = items.target(item);
+        direct_item_score<GRID, 3>(p, dk, patches[k], dk.cand, item, v, items.candidate(item, v),
+                                   direct_taps(p, dk, 0.0, 0.0, v, p.radius), j < fast_total, taps);
     }
     __syncthreads();
     if (!active) return;
-    warp_direct_aggregate(p, d, n);
+    warp_direct_aggregate<GRID>(p, d, n);
     bool seen = false;
     for (int c = lane; c <= n; c += 32) seen |= d.agg[c] == d.agg[c];
     const bool tested = __any_sync(0xffffffffu, seen);
