@@ -460,14 +460,22 @@ __global__ void __launch_bounds__(256, 4) direct_depth_kernel(DirectParams p) {
 // counter, since an entry's work depends on how many of its samples are inside their targets.
 // It waits for samples: what counts is how many warps an SM holds and how much of its memory is
 // left to the L1 cache. A copy of the taps (289 at the default radius, 8 bytes a target) is most
-// of a warp's shared memory, so from three targets on the taps are read from the tap lattice
-// (LATTICE), as lines that neighbouring nodes share. Measured on four targets: 15 warps an SM
-// with the copy and 32 without; direct stage at 4160x3120 14.05 -> 12.68 ms (retry 5.4 -> 4.1),
-// 1567x1173 with three targets 2.05 -> 1.96 ms. With one or two targets the copy fits beside as many
-// warps as the registers allow, and stays: reading the lattice there took 1.84 against 1.75 ms
-// (2080x1560, two targets) and 0.406 against 0.389 ms (1040x780, one).
+// of a warp's shared memory, so on a large grid, where it leaves an SM fewer than
+// WIDE_LATTICE_WARPS, the taps are read from the tap lattice (LATTICE), as lines that neighbouring
+// nodes share, in as many warps as the registers allow (32 of 64 registers with GRID, 24 of 80
+// without). Each of its entries takes longer, so a grid below WIDE_LATTICE_NODES keeps the copy, nine
+// taps in flight a lane: its list is a round or two of warps, whose latency counts. Direct stage,
+// copy / lattice, in ms: 400x300 (7,676 fine nodes), three targets at radius 4, 0.22 / 0.24, four at
+// radius 8, 0.81 / 1.02; 1200x900 (67,951) with four at radius 4 0.91 / 0.95; 1600x1200 (120,701) with
+// three 1.15 / 1.19; 2080x1560 (204,000), four targets with a narrow view, 3.01 / 2.92; 3200x2400
+// (481,000) with four 8.63 / 8.13; 4160x3120 (812,000) with four 14.77 / 13.77; 16640x1200 (1.25
+// million, without GRID) with four 21.3 / 19.8. With one or two targets at the default radius the copy
+// fits beside as many warps as the registers allow: 1.75 / 1.84 (2080x1560, two targets).
+constexpr size_t WIDE_LATTICE_NODES = 150000;
+constexpr int WIDE_LATTICE_WARPS = 24;
+
 template <bool GRID, bool LATTICE>
-__global__ void __launch_bounds__(256, LATTICE ? 0 : 3) direct_wide_kernel(DirectParams p) {
+__global__ void __launch_bounds__(256) direct_wide_kernel(DirectParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ RefPatch patches[8];
     const int slot = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -487,7 +495,7 @@ __global__ void __launch_bounds__(256, LATTICE ? 0 : 3) direct_wide_kernel(Direc
         warp_direct_candidates(p, cx, cy, d.cand, seeded);
         warp_stage_node(p, d, patch, cx, cy, p.wide_radius, p.spatial_wide, p.geometry + (size_t)node * V, nullptr);
         const int n = last - first + 1;
-        warp_direct_scores<GRID, LATTICE ? 4 : 3>(p, d, patch, d.cand + first, n, p.wide_radius, cx, cy);
+        warp_direct_scores<GRID, LATTICE ? 4 : 9>(p, d, patch, d.cand + first, n, p.wide_radius, cx, cy);
         double depth = 0.0;
         float confidence = 0.0f, improvement = 0.0f;
         int best;

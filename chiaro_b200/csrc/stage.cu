@@ -1937,14 +1937,13 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         p.nodes_per_cta = warps_per_cta(direct_kernel, slot, 8);
         direct_kernel<<<blocks_for(M, p.nodes_per_cta), 32 * p.nodes_per_cta, p.nodes_per_cta * slot, s>>>(p);
         CK(cudaGetLastError());
-        // the wide retry copies its taps unless that leaves an SM fewer warps than the registers do
+        // the wide retry copies its taps unless that leaves an SM too few warps on a large grid (direct_wide_kernel)
         auto wide_kernel = grid ? direct_wide_kernel<true, false> : direct_wide_kernel<false, false>;
         size_t wide_slot = direct_slot_bytes<float2>(V, wide_taps, WIDE_CANDIDATES);
-        int wide_warps = warps_per_cta(wide_kernel, wide_slot, 8), wide_blocks = 0, most_blocks = 0;
+        int wide_warps = warps_per_cta(wide_kernel, wide_slot, 8), wide_blocks = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wide_blocks, wide_kernel, 32 * wide_warps,
                                                          wide_warps * wide_slot));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&most_blocks, wide_kernel, 256, 0));
-        if (fine_lattice && wide_blocks * wide_warps < most_blocks * 8) {
+        if (fine_lattice && M >= WIDE_LATTICE_NODES && wide_blocks * wide_warps < WIDE_LATTICE_WARPS) {
             wide_kernel = grid ? direct_wide_kernel<true, true> : direct_wide_kernel<false, true>;
             wide_slot = direct_slot_bytes<NoTap>(V, wide_taps, WIDE_CANDIDATES);
             wide_warps = warps_per_cta(wide_kernel, wide_slot, 8);

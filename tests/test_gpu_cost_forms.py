@@ -77,8 +77,9 @@ def test_segments_far_beyond_the_reach_go_node_by_node(ctx):
         assert int(ctx.lib.chiaro_depth_tuning(ctx.handle, None, None, 0)) == n + 1
 
 
-# The luminance side at which no sample position is taken in f32 any more is 8192.
-@pytest.mark.parametrize("width,sources", [(16384, 1), (16400, 3)])
+# No sample position is taken in f32 beyond a luminance side of 8192. With three targets the grid of
+# 164,000 fine nodes is large enough for the wide retry to read its taps from the lattice.
+@pytest.mark.parametrize("width,sources", [(16384, 1), (16384, 3), (16400, 3)])
 def test_planes_beyond_the_f32_positions(ctx, width, sources):
     scene = make_case(width, 150, sources, 16, radius=3, focal=3000.0)
     assert compare_with_the_oracle(ctx, scene, direct=True).any()
