@@ -39,7 +39,6 @@ struct DecisionParams {
 };
 
 constexpr int DECISION_WARPS = 4;   // most nodes (warps) per CTA
-constexpr int DECISION_UNROLL = 4;  // taps in flight a lane
 
 // Per-warp shared memory of the decisions for V targets and T taps.
 struct DecisionSlot {
@@ -108,10 +107,11 @@ __device__ __forceinline__ int list_items(const DecisionSlot &d, int count, bool
 
 // The correlation of d's listed entry `at` (target v). The f64 form alone (zncc_any): a node
 // lists 24 or 32 items for one warp, so one item off the grid would cost the warp both loops.
+template <int UNROLL>
 __device__ __forceinline__ bool decision_score(const DecisionParams &p, const DecisionSlot &d, const RefPatch &patch,
                                                int at, int v, int taps, float &score) {
     const double2 dd = d.disp[at];
-    return zncc_any<DECISION_UNROLL>(p.views[p.targets[v]], d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y, score);
+    return zncc_any<UNROLL>(p.views[p.targets[v]], d.gh + v * taps, d.box[v], d.wt, patch, taps, dd.x, dd.y, score);
 }
 
 // Scores the pooled lists of the CTA's nodes (node k's count[k] entries of its
@@ -119,6 +119,7 @@ __device__ __forceinline__ bool decision_score(const DecisionParams &p, const De
 // correlations of one phase. Phase 1 items are (target, offset k < 5 or baseline
 // k = 5), phase 2 items (target, shift j < 8). A failed correlation of an offset
 // or shift marks its target's refinement as failed.
+template <int UNROLL>
 __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned char *smem_raw, size_t slot_bytes,
                                             const RefPatch *patches, const int *count, int nodes, int taps,
                                             bool shifts) {
@@ -132,7 +133,7 @@ __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned ch
         const int item = d.list[at];
         const int v = shifts ? item >> 3 : item / 6;
         float score;
-        const bool ok = decision_score(p, d, patches[k], at, v, taps, score);
+        const bool ok = decision_score<UNROLL>(p, d, patches[k], at, v, taps, score);
         const int kk = shifts ? 6 + (item & 7) : item - v * 6;
         if (ok)
             d.sc[v * 16 + kk] = score;
@@ -151,12 +152,22 @@ __device__ inline void decision_pool_scores(const DecisionParams &p, unsigned ch
 // The kernel waits for samples, so it wants warps: CTAs of four nodes with 64 registers give an SM
 // 32 of them (24 of 75 registers in CTAs of eight, whose barriers, or slots kept until the CTA is
 // done, also cost more). That leaves room for four taps in flight a lane instead of nine.
-// Measured, decisions: 4160x3120 with four targets 5.28 -> 4.72 ms, 3120x2340 with three 2.19 ->
+// Where the shared memory holds fewer than 32 warps' slots (DECISION_DEEP_SLOT), the 64 registers buy
+// none: nine taps in flight and up to 80 registers then (24 warps), on patches that fill rounds of
+// nine (DECISION_DEEP_TAPS). Decisions, four / nine taps, in ms: four targets at radius 4 1.64 / 1.56
+// (1800x1350), 4.70 / 4.19 (3200x2400), 8.30 / 7.07 (4160x3120), at radius 8 9.70 / 7.86; two at radius
+// 6 2.66 / 2.14; eight at radius 4 4.29 / 3.69; twelve 5.84 / 4.87 (4000x400). Below: three targets at
+// radius 4 (5.9 KB a slot) 3.98 / 4.13 (3200x2400), six at radius 3 (49 taps) 1.60 / 1.79 (1600x1200).
+// Measured, decisions of four taps: 4160x3120 with four targets 5.28 -> 4.72 ms, 3120x2340 with three 2.19 ->
 // 1.93, 1567x1173 with three 0.517 -> 0.501; pooled, 2080x1560 with two 1.021 -> 0.865, 1040x780
 // with one 0.378 -> 0.349. Without pooling, CTAs of two 4.67 / 1.98 / 0.517, of one 4.88 / 2.02 /
 // 0.526; 48 registers 5.69 ms.
-template <bool POOLED>
-__global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) target_decision_kernel(DecisionParams p) {
+constexpr int DECISION_DEEP_TAPS = 81;
+constexpr size_t DECISION_DEEP_SLOT = 7 * 1024;
+
+template <bool POOLED, int UNROLL>
+__global__ void __launch_bounds__(32 * DECISION_WARPS, UNROLL > 4 ? 6 : 8)
+    target_decision_kernel(DecisionParams p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ RefPatch patches[DECISION_WARPS];
     __shared__ int count[DECISION_WARPS];
@@ -239,7 +250,7 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) targ
     if constexpr (POOLED) {
         if (lane == 0) count[slot] = listed;
         __syncthreads();
-        decision_pool_scores(p, smem_raw, slot_bytes, patches, count, nodes, taps, false);
+        decision_pool_scores<UNROLL>(p, smem_raw, slot_bytes, patches, count, nodes, taps, false);
         __syncthreads();
     } else {
         __syncwarp();
@@ -247,7 +258,7 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) targ
             const int item = d.list[j];
             const int v = item / 6, k = item - v * 6;
             float score;
-            if (decision_score(p, d, patch, j, v, taps, score))
+            if (decision_score<UNROLL>(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + k] = score;
             else if (k < 5)
                 atomicOr(&d.flags[v], 1);
@@ -297,7 +308,7 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) targ
         __syncwarp();
         if (lane == 0) count[slot] = listed;
         __syncthreads();
-        decision_pool_scores(p, smem_raw, slot_bytes, patches, count, nodes, taps, true);
+        decision_pool_scores<UNROLL>(p, smem_raw, slot_bytes, patches, count, nodes, taps, true);
         __syncthreads();
     } else {
         __syncwarp();
@@ -305,7 +316,7 @@ __global__ void __launch_bounds__(32 * DECISION_WARPS, 32 / DECISION_WARPS) targ
             const int item = d.list[j];
             const int v = item >> 3;
             float score;
-            if (decision_score(p, d, patch, j, v, taps, score))
+            if (decision_score<UNROLL>(p, d, patch, j, v, taps, score))
                 d.sc[v * 16 + 6 + (item & 7)] = score;
             else
                 atomicOr(&d.flags[v], 1);

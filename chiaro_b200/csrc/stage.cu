@@ -291,8 +291,9 @@ void set_smem_limits() {
     for (auto kernel : {direct_depth_kernel<false>, direct_depth_kernel<true>, direct_wide_kernel<false, false>,
                         direct_wide_kernel<true, false>, direct_wide_kernel<false, true>, direct_wide_kernel<true, true>})
         CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(target_decision_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    CK(cudaFuncSetAttribute(target_decision_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    for (auto kernel : {target_decision_kernel<false, 4>, target_decision_kernel<true, 4>,
+                        target_decision_kernel<false, 9>, target_decision_kernel<true, 9>})
+        CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     CK(cudaFuncSetAttribute(align_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     done_devices.push_back(device);
 }
@@ -2044,7 +2045,9 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         if (slot > 200 * 1024) throw CudaError{cudaErrorInvalidValue, "decision shared memory exceeds 200 KiB"};
         // one or two targets leave most lanes of a node's warp idle in both phases (6 V and
         // 8 V items): the CTA then pools its nodes' correlations
-        const auto decision_kernel = V <= 2 ? target_decision_kernel<true> : target_decision_kernel<false>;
+        const bool deep = taps >= DECISION_DEEP_TAPS && slot > DECISION_DEEP_SLOT;
+        const auto decision_kernel = V <= 2 ? (deep ? target_decision_kernel<true, 9> : target_decision_kernel<true, 4>)
+                                            : (deep ? target_decision_kernel<false, 9> : target_decision_kernel<false, 4>);
         const int warps = warps_per_cta(decision_kernel, slot, DECISION_WARPS);
         decision_kernel<<<blocks_for(M, warps), 32 * warps, warps * slot, s>>>(p);
         CK(cudaGetLastError());
