@@ -52,8 +52,10 @@ struct CostParams {
     unsigned char passes[MAX_VIEWS];      // per target: parts that its labels are scored in
     TapLattice lattice;         // of this grid, or planes == nullptr
     int minimum_support, best_view_count;
+    int first_block;            // of the launch, in tiles
     float *view_scores;         // scratch [CTA][tile nodes][target][slot] of the launch
-    double2 *places;            // scratch [CTA (x, then y)][tile nodes * slots]
+    double2 *places;            // scratch [CTA (x, then y)][places_per_block]
+    int places_per_block;
     float *scores, *costs, *guidance;
     uint8_t *tested;
     // label subsets (slots == labels with no list and no bands: the full volume)
@@ -133,12 +135,13 @@ constexpr int TILE_NODES = 8;  // most nodes of a CTA
 // Node k of a tile CTA (-1: none) and its output row: consecutive entries of a node list, or a
 // block of the grid.
 __device__ __forceinline__ int tile_node(const CostParams &p, int n_rows, int k, int &row) {
+    const int tile = p.first_block + blockIdx.x;
     if (p.node_list) {
-        row = blockIdx.x * p.tile_w * p.tile_h + k;
+        row = tile * p.tile_w * p.tile_h + k;
         return row < n_rows ? __ldg(p.node_list + row) : -1;
     }
-    const int tiles_x = (p.columns + p.tile_w - 1) / p.tile_w, ty = blockIdx.x / tiles_x;
-    const int r = ty * p.tile_h + k / p.tile_w, c = (blockIdx.x - ty * tiles_x) * p.tile_w + k % p.tile_w;
+    const int tiles_x = (p.columns + p.tile_w - 1) / p.tile_w, ty = tile / tiles_x;
+    const int r = ty * p.tile_h + k / p.tile_w, c = (tile - ty * tiles_x) * p.tile_w + k % p.tile_w;
     row = r * p.columns + c;
     return r < p.rows && c < p.columns ? row : -1;
 }
@@ -221,8 +224,8 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
     const SmallDiv by_slots(D), by_pairs(pairs);
     const TileSmem s = carve_tile_smem(smem_raw, K, taps, D, p.region_rows);
     float *const score = p.view_scores + (size_t)blockIdx.x * K * V * D;  // [K][V][D], NaN = None
-    // displacements of the list's back
-    double2 *const places = p.places + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * K * D;
+    // displacements of the list's back, as many as the scratch holds
+    double2 *const places = p.places + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * p.places_per_block;
     const DevView &rv = p.views[p.reference];
     const TapLattice &lat = p.lattice;
 
@@ -364,7 +367,7 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
                     s.offset[fast_at] = offset;
                 } else if (scored) {
                     s.list[K * D - 1 - other_at] = (unsigned short)item;
-                    places[other_at] = make_double2(ddx, ddy);
+                    if (other_at < p.places_per_block) places[other_at] = make_double2(ddx, ddy);
                 }
             }
             if (__any_sync(full, span.x0 < INFINITY)) {
@@ -399,12 +402,12 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
                                  : zncc_region<false>(s.region, region, tap, patch[k], taps, s.offset[j], p.one, ok);
                 } else {
                     double2 at;
-                    if (fast) {  // the region does not fit: the displacement again
+                    if (!fast && j - n_fast < p.places_per_block) {
+                        at = places[j - n_fast];
+                    } else {  // the region does not fit, or the scratch is full: the displacement again
                         const int label = cost_slot_label(p, node_of[k], slot);
                         at = make_double2(0.0, 0.0);
                         if (label > 0) depth_delta(cam, geom[k], p.label_depth[label], at.x, at.y);
-                    } else {
-                        at = places[j - n_fast];
                     }
                     const double2 place = make_double2(at.x * 0.5, at.y * 0.5);
                     if (fits && taps_inside(tap_range(box[k], place.x, place.y), tv.luma.width, tv.luma.height))

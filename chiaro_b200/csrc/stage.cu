@@ -352,6 +352,24 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
     }
 }
 
+// The scratch of a cost volume in tiles, a word per item and target: a buffer that later passes write
+// and that is free until the volume is done (the SGM's eight paths), so it costs no memory. Where it
+// holds less than the whole volume (the SGM's: from eight targets on, or fewer on a grid that tiles
+// cover badly) the tiles go in several launches. What it holds beyond the scores keeps displacements
+// of off-grid items (all of them up to three targets, part of them above); computing each again takes
+// 2% of the volume's time (coarse search of 2080x1560, three targets: 2.57 against 2.52 ms).
+struct CostScratch {
+    float *data;
+    size_t floats;
+};
+
+// Floats of one of the SGM's eight path planes, and the buffer of all of them.
+size_t sgm_pitch(size_t total) { return (total + 63) / 64 * 64; }
+
+CostScratch sgm_path_planes(chiaro_depth_ctx *ctx, size_t total) {
+    return {dbuf<float>(ctx, "sgm_paths", 8 * sgm_pitch(total)), 8 * sgm_pitch(total)};
+}
+
 // Launch build_cost_volume over n_rows nodes. With autotuning on, the first launch of a
 // (targets, labels scored, radius) bucket in a form of the kernel (node by node, or in tiles of
 // so many nodes, targets in turn or side by side) large enough to time (at least 4096 nodes,
@@ -361,12 +379,12 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
 // below writes the outputs again.
 constexpr uint64_t COST_BUCKET_MASK = ((uint64_t)1 << 40) - 1;  // of a key: its bucket; the form lies above
 void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView> &views, size_t n_rows,
-                 size_t path_floats) {
+                 const CostScratch &scratch) {
     cudaStream_t s = ctx->stream;
     const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
     const bool tiles = p.patches != nullptr;
     size_t smem = node_form_bytes(p.n_targets, taps, p.slots);
-    unsigned blocks = (unsigned)n_rows, turns = 1;
+    unsigned blocks = (unsigned)n_rows, turns = 1, chunk = blocks;
     if (tiles) {
         plan_cost_tiles(p, views, n_rows, ctx->sm_count);
         const int nodes = p.tile_w * p.tile_h;
@@ -375,18 +393,32 @@ void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView>
                                         : div_ceil(p.columns, p.tile_w) * div_ceil(p.rows, p.tile_h));
         // a grid of less than two waves of CTAs (seven an SM): a CTA per target
         if (p.n_targets > 1 && blocks < 14u * ctx->sm_count) turns = (unsigned)p.n_targets;
-        // the launch's scratch shares the SGM's path buffers, which are free until the volume is done
-        const size_t items = (size_t)blocks * nodes * p.slots;
-        float *scratch = dbuf<float>(ctx, "sgm_paths", std::max(items * (4 * turns + p.n_targets), path_floats));
-        p.places = reinterpret_cast<double2 *>(scratch);
-        p.view_scores = scratch + 4 * items * turns;
+        const size_t block_floats = (size_t)nodes * p.slots * p.n_targets;
+        if (scratch.floats < block_floats)
+            throw CudaError{cudaErrorInvalidValue, "cost volume: the scratch holds less than one tile"};
+        p.view_scores = scratch.data;
+        chunk = (unsigned)std::min<size_t>(blocks, scratch.floats / block_floats);
+        chunk = (unsigned)div_ceil(blocks, div_ceil(blocks, chunk));  // of equal size
+        const size_t score_floats = (chunk * block_floats + 3) / 4 * 4;  // places lie on 16 bytes
+        p.places = reinterpret_cast<double2 *>(scratch.data + score_floats);
+        if (scratch.floats > score_floats)
+            p.places_per_block = (int)std::min<size_t>((scratch.floats - score_floats) / 4 / ((size_t)chunk * turns),
+                                                       (size_t)nodes * p.slots);
+        ctx->launches += (int)(div_ceil(blocks, chunk) * (turns > 1 ? 2 : 1)) - 1;
     }
     const auto launch = [&](int threads) {
-        if (tiles)
-            cost_kernel_for(threads)<<<dim3(blocks, turns), threads, smem, s>>>(p, (int)n_rows);
-        else
+        if (!tiles) {
             cost_node_kernel_for(threads)<<<blocks, threads, smem, s>>>(p);
-        CK(cudaGetLastError());
+            CK(cudaGetLastError());
+            return;
+        }
+        for (unsigned first = 0; first < blocks; first += chunk) {
+            const unsigned count = std::min(chunk, blocks - first);
+            p.first_block = (int)first;
+            cost_kernel_for(threads)<<<dim3(count, turns), threads, smem, s>>>(p, (int)n_rows);
+            if (turns > 1) cost_aggregate_kernel<<<count, 128, 0, s>>>(p, (int)n_rows);
+            CK(cudaGetLastError());
+        }
     };
     const uint64_t form = tiles ? (uint64_t)(p.tile_w * p.tile_h) << 1 | (turns > 1 ? 1 : 0) : 0;
     const uint64_t key =
@@ -423,11 +455,6 @@ void launch_cost(chiaro_depth_ctx *ctx, CostParams p, const std::vector<DevView>
         ctx->cost_tuning[key] = threads;
     }
     launch(threads);
-    if (turns > 1) {
-        cost_aggregate_kernel<<<blocks, 128, 0, s>>>(p, (int)n_rows);
-        CK(cudaGetLastError());
-        ctx->launches += 1;
-    }
 }
 
 // Per (node, target) geometry records of one or two step-spaced grids.
@@ -511,8 +538,8 @@ void launch_sgm(chiaro_depth_ctx *ctx, const float *data, const float *guidance,
                 int labels) {
     const int K = (labels + 31) / 32;  // label sets per lane
     const size_t total = (size_t)columns * rows * labels;
-    const size_t pitch = (total + 63) / 64 * 64;
-    float *paths = dbuf<float>(ctx, "sgm_paths", 8 * pitch);
+    const size_t pitch = sgm_pitch(total);
+    float *paths = sgm_path_planes(ctx, total).data;
     switch (K) {
 #define SGM_CASE(k)                                                         \
     case k:                                                                 \
@@ -1248,8 +1275,8 @@ struct CoarseGrid {
 };
 
 void coarse_cost(chiaro_depth_ctx *ctx, const CoarseGrid &g, int reference, const chiaro_depth_options &o, int slots,
-                 const int *label_list, const BandGrid *band, const int *node_list, size_t n_rows, float *scores,
-                 float *costs, float *guidance, uint8_t *tested) {
+                 const int *label_list, const BandGrid *band, const int *node_list, size_t n_rows,
+                 const CostScratch &scratch, float *scores, float *costs, float *guidance, uint8_t *tested) {
     if (n_rows == 0) return;
     CostParams p{};
     p.geometry = g.geometry;
@@ -1284,7 +1311,7 @@ void coarse_cost(chiaro_depth_ctx *ctx, const CoarseGrid &g, int reference, cons
     const int taps = (2 * p.radius + 1) * (2 * p.radius + 1);
     if ((size_t)g.V * slots > 65535 || node_smem_bytes(g.V, taps, slots) > 200 * 1024)
         throw CudaError{cudaErrorInvalidValue, "cost volume: targets x labels exceed the node CTA's shared memory"};
-    launch_cost(ctx, p, g.h_views, n_rows, 0);
+    launch_cost(ctx, p, g.h_views, n_rows, scratch);
 }
 
 // The coarse search of the stage's reference grid (depth.rs:1187-1467 up to the winner):
@@ -1358,7 +1385,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         CK(cudaEventRecord(ctx->events[2], s));
         CK(cudaEventRecord(ctx->events[3], s));
         float *scores = dbuf<float>(ctx, "coarse.scores", N * D), *costs = dbuf<float>(ctx, "coarse.costs", N * D);
-        coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, nullptr, N, scores, costs, guidance, tested);
+        coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, nullptr, N, sgm_path_planes(ctx, N * D), scores, costs, guidance, tested);
         CK(cudaEventRecord(ctx->events[4], s));
         float *aggregate = dbuf<float>(ctx, "coarse.aggregate", N * D);
         launch_sgm(ctx, costs, guidance, aggregate, g.columns, g.rows, D);
@@ -1377,8 +1404,8 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         upload(ctx, d_list, list.data(), PREPASS_SLOTS);
         float *pre_scores = dbuf<float>(ctx, "coarse.prepass_scores", N * PREPASS_SLOTS);
         float *pre_costs = dbuf<float>(ctx, "coarse.prepass_costs", N * PREPASS_SLOTS);
-        coarse_cost(ctx, g, reference, o, PREPASS_SLOTS, d_list, nullptr, nullptr, N, pre_scores, pre_costs, guidance,
-                    tested);
+        coarse_cost(ctx, g, reference, o, PREPASS_SLOTS, d_list, nullptr, nullptr, N, {}, pre_scores, pre_costs,
+                    guidance, tested);
         CK(cudaEventRecord(ctx->events[2], s));
         if (prepass_out) {
             CK(cudaMemcpyAsync(prepass_out, pre_costs, N * PREPASS_SLOTS * sizeof(float), cudaMemcpyDeviceToDevice, s));
@@ -1409,7 +1436,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         float *band_costs = dbuf<float>(ctx, "coarse.band_costs", N * (1 + band));
         uint8_t *band_tested = dbuf<uint8_t>(ctx, "coarse.band_tested", N);
         float *band_guidance = dbuf<float>(ctx, "coarse.band_guidance", N);
-        coarse_cost(ctx, g, reference, o, 1 + band, nullptr, &grid, nullptr, N, band_scores, band_costs,
+        coarse_cost(ctx, g, reference, o, 1 + band, nullptr, &grid, nullptr, N, {}, band_scores, band_costs,
                     band_guidance, band_tested);
         CK(cudaEventRecord(ctx->events[4], s));
         // the banded SGM, its winners, the edge and cross-view fallback flags
@@ -1466,9 +1493,12 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
             uint8_t *wtested = dbuf<uint8_t>(ctx, "coarse.window_tested", node_count);
             float *wagg = dbuf<float>(ctx, "coarse.window_aggregate", cost_floats);
             full_range_patches();
-            coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, d_nodes, node_count, wscores, wcosts, wguid,
-                        wtested);
-            if (windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows) {
+            const bool whole = windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows;
+            // the band's paths are done with
+            const CostScratch scratch = whole ? sgm_path_planes(ctx, N * D) : CostScratch{paths, 8 * pitch};
+            coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, d_nodes, node_count, scratch, wscores, wcosts,
+                        wguid, wtested);
+            if (whole) {
                 launch_sgm(ctx, wcosts, wguid, wagg, g.columns, g.rows, D);
             } else {
                 std::vector<chiaro_sgm_instance> instances(windows.size());
@@ -1835,7 +1865,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         int taps = (2 * radius + 1) * (2 * radius + 1);
         if ((size_t)V * D > 65535 || node_smem_bytes(V, taps, D) > 200 * 1024)
             throw CudaError{cudaErrorInvalidValue, "cost volume: targets x labels exceed the node CTA's shared memory"};
-        launch_cost(ctx, p, h_views, N, 8 * ((N * D + 63) / 64 * 64));
+        launch_cost(ctx, p, h_views, N, sgm_path_planes(ctx, N * D));
     }
     record_event(ctx->events[1], s, capturing);
     // ---- SGM

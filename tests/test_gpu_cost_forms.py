@@ -83,3 +83,26 @@ def test_segments_far_beyond_the_reach_go_node_by_node(ctx):
 def test_planes_beyond_the_f32_positions(ctx, width, sources):
     scene = make_case(width, 150, sources, 16, radius=3, focal=3000.0)
     assert compare_with_the_oracle(ctx, scene, direct=True).any()
+
+
+@pytest.mark.parametrize("width,height,sources,planes", [(700, 520, 2, 96), (700, 520, 4, 96), (700, 520, 12, 96),
+                                                        (1000, 700, 9, 40)])
+def test_tiles_hold_no_scratch_of_their_own(width, height, sources, planes):
+    """The same call with a lens that takes the tiles and with one that does not: the tiles add the
+    nodes' reference patches (24 bytes each) and at most a copy of the targets' planes, and go in
+    several launches from eight targets on, side by side (700x520) or in turn."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from chiaro_b200.runtime import DepthContext
+    held = []
+    for focal in (1200.0, 15000.0):
+        scene = make_case(width, height, sources, planes, focal=focal)
+        context = DepthContext(0)
+        try:
+            assert compare_with_the_oracle(context, scene).any()
+            held.append(context.memory_held())
+        finally:
+            context.close()
+    _, (cc, cr, _) = output_shape(width, height, scene.options)
+    assert 0 < held[0] - held[1] <= 24 * cc * cr + sources * 4 * (width // 2 + 3) * (height // 2 + 3)
