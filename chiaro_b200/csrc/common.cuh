@@ -559,7 +559,8 @@ struct DevView {
     PlaneRef luma;
     const float4 *quads;  // bilinear neighbourhood (quad) plane of the luminance (targets only)
     int quad_stride;      // of its rows, in quads (quad_index)
-    PaddedPlane rows_plane, columns_plane;  // the luminance and its transpose (targets only)
+    PaddedPlane region_plane;  // the luminance, or its transpose (targets of node tiles only)
+    int region_transposed;
     WarpRef warp;
     int width, height;
     int has_camera, accepted;

@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
             const bool transposed = p.transposed[v];
             Region region;
             const bool fits = range[0] != INT32_MAX && region_of(range, transposed, p.region_rows, region);
-            if (fits) load_region(region, transposed ? tv.columns_plane : tv.rows_plane, s.region, tid, T);
+            if (fits) load_region(region, tv.region_plane, s.region, tid, T);
             copy_async_wait();
             __syncthreads();
             // ---- the correlations of the listed items

@@ -69,6 +69,9 @@ struct chiaro_depth_ctx {
     int union_retries = -1;
     uint64_t memory_limit = 0;
     uint64_t memory_held = 0;
+    // cost volumes of this many hypotheses or more go node by node, since one of so many could not
+    // hold the node tiles' buffers (with_tiles_that_fit); and the tiles' hypotheses of the present call
+    size_t tiles_refused = SIZE_MAX, tiles_taken = 0;
     // launch shapes chosen by the autotuner: cost-volume threads per CTA per bucket and form
     // (launch_cost); autotune: 1 tune, 0 the default shape, or a forced shape (threads per CTA)
     int autotune = 1;
@@ -88,19 +91,46 @@ struct CudaError {
         if (e_ != cudaSuccess) throw CudaError{e_, #call};         \
     } while (0)
 
-// Grow-only named device buffer of at least `count` elements.
+// Frees the buffers that only the cost volume's node tiles read (region_planes, the coarse nodes'
+// patches). True if there were any.
+bool drop_tile_buffers(chiaro_depth_ctx *ctx) {
+    bool any = false;
+    for (auto &[name, b] : ctx->buffers) {
+        if (!b.ptr || (name.rfind("region", 0) != 0 && name != "coarse_patches")) continue;
+        CK(cudaFree(b.ptr));
+        ctx->memory_held -= b.bytes;
+        b = {};
+        ++ctx->alloc_epoch;
+        any = true;
+    }
+    return any;
+}
+
+// Grow-only named device buffer of at least `count` elements. Buffers of node tiles that the present
+// call does not use make room for it.
 template <class T>
 T *dbuf(chiaro_depth_ctx *ctx, const std::string &name, size_t count) {
     size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
     auto &b = ctx->buffers[name];
     if (b.bytes < bytes) {
-        if (ctx->memory_limit && ctx->memory_held - b.bytes + bytes > ctx->memory_limit)
+        const auto refused = [&] {
+            return ctx->memory_limit && ctx->memory_held - b.bytes + bytes > ctx->memory_limit;
+        };
+        if (refused() && (ctx->tiles_taken || !drop_tile_buffers(ctx) || refused()))
             throw CudaError{cudaErrorMemoryAllocation, "a context buffer beyond the context's memory limit"};
         if (b.ptr) CK(cudaFree(b.ptr));
         ctx->memory_held -= b.bytes;
         b.ptr = nullptr;
         b.bytes = 0;
-        CK(cudaMalloc(&b.ptr, bytes));
+        cudaError_t status = cudaMalloc(&b.ptr, bytes);
+        if (status == cudaErrorMemoryAllocation && !ctx->tiles_taken && drop_tile_buffers(ctx)) {
+            cudaGetLastError();
+            status = cudaMalloc(&b.ptr, bytes);
+        }
+        if (status != cudaSuccess) {
+            b.ptr = nullptr;
+            throw CudaError{status, "cudaMalloc of a context buffer"};
+        }
         b.bytes = bytes;
         ctx->memory_held += bytes;
         ++ctx->alloc_epoch;  // a captured stage graph holding the old pointer is void
@@ -252,9 +282,10 @@ bool epipolar_extent(const DevView &rv, const DevView &tv, double near_depth, do
 constexpr size_t COST_TILE_LARGE_GRID = 40000;
 constexpr double COST_TILE_SEGMENTS[] = {1000.0, 1300.0, 2000.0};  // small grid; large; large, at most three targets
 
-bool cost_in_tiles(const std::vector<DevView> &views, int reference, const std::vector<int> &targets, double near_depth,
-                   size_t nodes, int labels) {
-    if (nodes * targets.size() * labels < COST_TILE_ITEMS) return false;
+bool cost_in_tiles(chiaro_depth_ctx *ctx, const std::vector<DevView> &views, int reference,
+                   const std::vector<int> &targets, double near_depth, size_t nodes, int labels) {
+    const size_t items = nodes * targets.size() * labels;
+    if (items < COST_TILE_ITEMS || items >= ctx->tiles_refused) return false;
     int side = 0;
     double segments = 0.0, dx, dy;
     for (int t : targets) {
@@ -262,7 +293,37 @@ bool cost_in_tiles(const std::vector<DevView> &views, int reference, const std::
         if (epipolar_extent(views[reference], views[t], near_depth, dx, dy)) segments += std::max(dx, dy);
     }
     const int grid = nodes < COST_TILE_LARGE_GRID ? 0 : targets.size() > 3 ? 1 : 2;
-    return side >= COST_TILE_SIDE && segments <= COST_TILE_SEGMENTS[grid];
+    if (side < COST_TILE_SIDE || segments > COST_TILE_SEGMENTS[grid]) return false;
+    ctx->tiles_taken = items;
+    return true;
+}
+
+// Runs a call. Where memory or the context's limit does not hold it with the node tiles' buffers, it
+// runs again without them: every call that fits node by node is answered, with the same bits.
+template <typename Call>
+auto with_tiles_that_fit(chiaro_depth_ctx *ctx, const Call &call) {
+    struct Taken {  // the tiles' buffers are in use until the call ends
+        size_t &taken;
+        ~Taken() { taken = 0; }
+    } taken{ctx->tiles_taken};
+    try {
+        return call();
+    } catch (const CudaError &e) {
+        if (e.code != cudaErrorMemoryAllocation || !ctx->tiles_taken) throw;
+    }
+    cudaGetLastError();
+    CK(cudaStreamSynchronize(ctx->copy_stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    const size_t before = ctx->tiles_refused;
+    ctx->tiles_refused = ctx->tiles_taken;
+    ctx->tiles_taken = 0;
+    drop_tile_buffers(ctx);
+    try {
+        return call();
+    } catch (const CudaError &) {
+        ctx->tiles_refused = before;  // not the tiles' fault
+        throw;
+    }
 }
 
 CostKernel cost_kernel_for(int threads) {
@@ -330,11 +391,10 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
     const DevView &rv = views[p.reference];
     for (int v = 0; v < p.n_targets; ++v) {
         const DevView &tv = views[p.targets[v]];
-        p.transposed[v] = 0;
+        p.transposed[v] = tv.region_transposed != 0;
         p.passes[v] = 1;
         double dx, dy;
         if (!epipolar_extent(rv, tv, p.near_depth, dx, dy)) continue;
-        p.transposed[v] = dy > dx;
         // the share of the segment that the scored labels cover, and the room for it beside the
         // patch, the tile's nodes, the bilinear neighbour, alignment and the warp's own bending
         const double share = p.band_first ? (double)p.slots / p.labels : 1.0;
@@ -475,23 +535,34 @@ void launch_geometry(chiaro_depth_ctx *ctx, const DevView *d_views, int referenc
     CK(cudaGetLastError());
 }
 
-// The buffers of a target's planes for the correlations: quads, padded rows, padded columns.
-void sample_planes(chiaro_depth_ctx *ctx, int t, DevView &v) {
-    const PlaneRef &lp = v.luma;
-    const std::string name = std::to_string(t);
-    v.quad_stride = quad_stride(lp.width);
-    v.quads = dbuf<float4>(ctx, "quads" + name, quad_count(lp.width, lp.height));
-    v.rows_plane.pitch = (lp.width + 3) / 4 * 4;
-    v.rows_plane.data = dbuf<float>(ctx, "rows" + name, (size_t)v.rows_plane.pitch * lp.height);
-    v.columns_plane.pitch = (lp.height + 3) / 4 * 4;
-    v.columns_plane.data = dbuf<float>(ctx, "columns" + name, (size_t)v.columns_plane.pitch * lp.width);
+// The buffer of a target's quad plane.
+void quad_plane(chiaro_depth_ctx *ctx, int t, DevView &v) {
+    v.quad_stride = quad_stride(v.luma.width);
+    v.quads = dbuf<float4>(ctx, "quads" + std::to_string(t), quad_count(v.luma.width, v.luma.height));
 }
 
+// The buffers of the planes that the node tiles copy their regions from: rows along the axis nearer
+// to the target's epipolar segment.
+void region_planes(chiaro_depth_ctx *ctx, std::vector<DevView> &views, int reference, const std::vector<int> &targets,
+                   double near_depth) {
+    for (int t : targets) {
+        DevView &v = views[t];
+        double dx, dy;
+        v.region_transposed = epipolar_extent(views[reference], v, near_depth, dx, dy) && dy > dx;
+        const size_t length = v.region_transposed ? v.luma.height : v.luma.width;
+        const size_t rows = v.region_transposed ? v.luma.width : v.luma.height;
+        v.region_plane.pitch = (int)((length + 3) / 4 * 4);
+        v.region_plane.data = dbuf<float>(ctx, "region" + std::to_string(t), v.region_plane.pitch * rows);
+    }
+}
+
+// Writes the targets' planes: the quad planes (if `quads`) and those of region_planes.
 void launch_sample_planes(chiaro_depth_ctx *ctx, const DevView *d_views, const std::vector<DevView> &views,
-                          const std::vector<int> &targets) {
+                          const std::vector<int> &targets, bool quads) {
     if (targets.empty()) return;
     PlanesParams p{};
     p.views = d_views;
+    p.quads = quads;
     size_t most = 0;
     for (size_t v = 0; v < targets.size(); ++v) {
         const PlaneRef &lp = views[targets[v]].luma;
@@ -1344,7 +1415,10 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     g.spatial = dbuf<float>(ctx, "coarse.spatial", sp.size());
     upload(ctx, g.labels, labels.data(), D);
     upload(ctx, g.spatial, sp.data(), sp.size());
-    for (int t : g.targets) sample_planes(ctx, t, h_views[t]);
+    for (int t : g.targets) quad_plane(ctx, t, h_views[t]);
+    // the node tiles of a full-range cost volume; a banded search decides it for its fallback windows
+    bool in_tiles = !spec && cost_in_tiles(ctx, h_views, reference, g.targets, o.near_depth, N, D);
+    if (in_tiles) region_planes(ctx, h_views, reference, g.targets, o.near_depth);
     g.views = dbuf<DevView>(ctx, "coarse.views", n_views);
     upload(ctx, g.views, h_views.data(), n_views);
     g.geometry = dbuf<GeomRec>(ctx, "coarse_geometry", N * std::max(g.V, 1));
@@ -1369,14 +1443,13 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
         tap_lattice_kernel<<<blocks_for((size_t)g.lattice.columns * g.lattice.rows, 256), 256, 0, s>>>(p);
         CK(cudaGetLastError());
     }
-    launch_sample_planes(ctx, g.views, h_views, g.targets);
+    launch_sample_planes(ctx, g.views, h_views, g.targets, true);
     g.h_views = h_views;
-    const auto full_range_patches = [&] {  // the node tiles of a full-range cost volume read them
-        if (!cost_in_tiles(h_views, reference, g.targets, o.near_depth, N, D)) return;
+    const auto tile_patches = [&] {
         g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
         launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
     };
-    if (!spec) full_range_patches();
+    if (in_tiles) tile_patches();
     CK(cudaEventRecord(ctx->events[1], s));
     uint8_t *tested = dbuf<uint8_t>(ctx, "coarse.tested", N);
     float *guidance = dbuf<float>(ctx, "coarse.guidance", N);
@@ -1492,7 +1565,14 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
             float *wguid = dbuf<float>(ctx, "coarse.window_guidance", node_count);
             uint8_t *wtested = dbuf<uint8_t>(ctx, "coarse.window_tested", node_count);
             float *wagg = dbuf<float>(ctx, "coarse.window_aggregate", cost_floats);
-            full_range_patches();
+            in_tiles = cost_in_tiles(ctx, h_views, reference, g.targets, o.near_depth, N, D);
+            if (in_tiles) {
+                region_planes(ctx, h_views, reference, g.targets, o.near_depth);
+                upload(ctx, g.views, h_views.data(), n_views);
+                launch_sample_planes(ctx, g.views, h_views, g.targets, false);
+                g.h_views = h_views;
+                tile_patches();
+            }
             const bool whole = windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows;
             // the band's paths are done with
             const CostScratch scratch = whole ? sgm_path_planes(ctx, N * D) : CostScratch{paths, 8 * pitch};
@@ -1725,8 +1805,10 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     float *d_sp = reinterpret_cast<float *>(d_labels + doubles), *d_sp_direct = d_sp + sp.size();
     float *d_sp_wide = d_sp_direct + sp_direct.size();
     upload(ctx, d_labels, tables.data(), tables.size());
-    // the quad planes' buffers and the views that point at them, before any launch
-    for (int t : targets) sample_planes(ctx, t, h_views[t]);
+    // the planes' buffers and the views that point at them, before any launch
+    for (int t : targets) quad_plane(ctx, t, h_views[t]);
+    const bool tiles = cost_in_tiles(ctx, h_views, reference, targets, o.near_depth, N, D);
+    if (tiles) region_planes(ctx, h_views, reference, targets, o.near_depth);
     upload(ctx, d_views, h_views.data(), h_views.size());
     GeomRec *coarse_geometry = dbuf<GeomRec>(ctx, "coarse_geometry", N * std::max(V, 1));
     GeomRec *fine_geometry = dbuf<GeomRec>(ctx, "fine_geometry", M * std::max(V, 1));
@@ -1824,15 +1906,15 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
     RefPatch *coarse_patches = nullptr;  // the node tiles of the cost volume read them
     std::vector<PatchGrid> patch_grids{{(int)g.columns, (int)g.rows, (int)g.step, direct_radius, d_sp_direct,
                                         fine_lattice ? lattice : TapLattice{}, fine_patches}};
-    if (cost_in_tiles(h_views, reference, targets, o.near_depth, N, D)) {
+    if (tiles) {
         coarse_patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
         patch_grids.push_back({(int)g.coarse_columns, (int)g.coarse_rows, (int)g.coarse_step, radius, d_sp,
                                coarse_lattice ? lattice : TapLattice{}, coarse_patches});
     }
     launch_patches(ctx, d_views, reference, patch_grids);
     if (host_planes) CK(cudaStreamWaitEvent(s, ctx->planes_ready, 0));
-    // quad planes of the target luminance for the fast ZNCC path
-    launch_sample_planes(ctx, d_views, h_views, targets);
+    // the planes of the target luminance that the correlations read
+    launch_sample_planes(ctx, d_views, h_views, targets, true);
     // ---- cost volume
     float *scores = dbuf<float>(ctx, "scores", N * D);
     float *costs = dbuf<float>(ctx, "costs", N * D);
@@ -2271,8 +2353,11 @@ int refine(chiaro_depth_ctx *ctx, const chiaro_view *views, size_t n_views, size
         Results *d_results = dbuf<Results>(ctx, "results", 1);
         Results h_results{};
         std::vector<int> rewritten;
-        run_stage(ctx, h_views, d_views, (int)reference_index, o, g, out, d_results, h_results, debug, rewritten,
-                  device_pointers ? nullptr : &host);
+        with_tiles_that_fit(ctx, [&] {
+            rewritten.clear();
+            run_stage(ctx, h_views, d_views, (int)reference_index, o, g, out, d_results, h_results, debug, rewritten,
+                      device_pointers ? nullptr : &host);
+        });
         out_map->columns = g.columns;
         out_map->rows = g.rows;
         out_map->step = g.step;
@@ -2434,6 +2519,8 @@ int chiaro_depth_set_union_retry_limit(chiaro_depth_ctx *ctx, int32_t retries) {
 int chiaro_depth_set_memory_limit(chiaro_depth_ctx *ctx, uint64_t bytes) {
     if (!ctx) return CHIARO_ERR_ARGUMENT;
     ctx->memory_limit = bytes;
+    if (ctx->tiles_refused != SIZE_MAX) ++ctx->alloc_epoch;  // a captured stage graph may be of the other form
+    ctx->tiles_refused = SIZE_MAX;
     return CHIARO_OK;
 }
 
@@ -2837,8 +2924,10 @@ int chiaro_coarse_depth_device(chiaro_depth_ctx *ctx, const chiaro_view *views, 
     }
     try {
         CK(cudaSetDevice(ctx->device));
-        return run_coarse(ctx, h_views, (int)reference_index, *options, band ? &spec : nullptr, winner, tested,
-                          tile_offsets, tile_fallback, report, nullptr, nullptr);
+        return with_tiles_that_fit(ctx, [&] {
+            return run_coarse(ctx, h_views, (int)reference_index, *options, band ? &spec : nullptr, winner, tested,
+                              tile_offsets, tile_fallback, report, nullptr, nullptr);
+        });
     } catch (const CudaError &e) {
         return fail(ctx, e);
     }

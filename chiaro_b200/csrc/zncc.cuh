@@ -556,12 +556,14 @@ __device__ __forceinline__ size_t quad_index(int x, int y, int stride) {
     return (size_t)(y >> 1) * stride + 2 * x + (y & 1);
 }
 
-// Every target's planes for the correlations, in one launch: the quad plane, and for load_region
-// the plane and its transpose with rows padded to a multiple of 4 floats. A CTA of 32 x 8
-// threads makes a 32 x 32 tile of target blockIdx.y from one read of it and its right and lower
-// neighbours. HBM-bound: 4 B read, 24 B written per pixel.
+// Every target's planes for the correlations, in one launch: the quad plane, and where the cost
+// volume runs in node tiles the plane or its transpose (region_transposed) with rows padded to a
+// multiple of 4 floats, for load_region. A CTA of 32 x 8 threads makes a 32 x 32 tile of target
+// blockIdx.y from one read of it and its right and lower neighbours. HBM-bound: 4 B read, 16 B
+// written per pixel, and 4 B more for the tiles.
 struct PlanesParams {
     const DevView *views;
+    int quads;  // whether the quad planes are written
     int targets[MAX_VIEWS];
 };
 
@@ -578,17 +580,19 @@ __global__ void __launch_bounds__(256) sample_planes_kernel(PlanesParams p) {
     }
     __syncthreads();
     float4 *quads = const_cast<float4 *>(v.quads);
-    float *rows = const_cast<float *>(v.rows_plane.data), *columns = const_cast<float *>(v.columns_plane.data);
+    float *const region = const_cast<float *>(v.region_plane.data);
+    const bool rows = region && !v.region_transposed, columns = region && v.region_transposed;
     for (int r = threadIdx.y; r < 32; r += 8) {
         int x = x0 + lane, y = y0 + r;
         if (x < width && y < height) {
-            rows[(size_t)y * v.rows_plane.pitch + x] = tile[r][lane];
-            quads[quad_index(x, y, v.quad_stride)] =
-                make_float4(tile[r][lane], tile[r][lane + 1], tile[r + 1][lane], tile[r + 1][lane + 1]);
+            if (rows) region[(size_t)y * v.region_plane.pitch + x] = tile[r][lane];
+            if (p.quads)
+                quads[quad_index(x, y, v.quad_stride)] =
+                    make_float4(tile[r][lane], tile[r][lane + 1], tile[r + 1][lane], tile[r + 1][lane + 1]);
         }
         x = x0 + r;
         y = y0 + lane;
-        if (x < width && y < height) columns[(size_t)x * v.columns_plane.pitch + y] = tile[lane][r];
+        if (columns && x < width && y < height) region[(size_t)x * v.region_plane.pitch + y] = tile[lane][r];
     }
 }
 

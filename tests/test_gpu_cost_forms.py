@@ -106,3 +106,36 @@ def test_tiles_hold_no_scratch_of_their_own(width, height, sources, planes):
             context.close()
     _, (cc, cr, _) = output_shape(width, height, scene.options)
     assert 0 < held[0] - held[1] <= 24 * cc * cr + sources * 4 * (width // 2 + 3) * (height // 2 + 3)
+
+
+@pytest.mark.parametrize("sources", [2, 9])
+def test_a_limit_that_holds_the_other_form_is_enough(sources):
+    """A context whose memory limit holds the call node by node answers it, with the same bits, first
+    and again, after a call of another size took the tiles, and in tiles when the limit is lifted."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from chiaro_b200.runtime import DepthContext
+    tiled, nodewise = (make_case(1000, 700, sources, 40, focal=focal) for focal in (1200.0, 15000.0))
+    smaller = make_case(900, 640, sources, 40, focal=1200.0)
+    results, held = [], []
+    for scene, limit in ((nodewise, False), (tiled, False), (tiled, True)):
+        context = DepthContext(0)
+        try:
+            if limit:
+                context.set_memory_limit(held[0])
+                run(context, smaller)
+            for _ in range(2 if limit else 1):
+                results.append(run(context, scene)[0])
+            held.append(context.memory_held())
+            if limit:
+                assert held[-1] <= held[0]
+                context.set_memory_limit(0)
+                results.append(run(context, scene)[0])
+                assert context.memory_held() > held[0]
+        finally:
+            context.close()
+    assert held[1] > held[0]
+    for other in results[2:]:
+        assert np.array_equal(other.depth.view(np.uint64), results[1].depth.view(np.uint64))
+        assert np.array_equal(other.confidence.view(np.uint32), results[1].confidence.view(np.uint32))
