@@ -581,7 +581,7 @@ void launch_patches(chiaro_depth_ctx *ctx, const DevView *d_views, int reference
     size_t most = 0;
     for (size_t i = 0; i < grids.size(); ++i) {
         p.grids[i] = grids[i];
-        most = std::max(most, (size_t)grids[i].columns * grids[i].rows);
+        most = std::max(most, grids[i].nodes ? (size_t)grids[i].listed : (size_t)grids[i].columns * grids[i].rows);
     }
     patch_sums_kernel<<<dim3(blocks_for(most, 256), (unsigned)grids.size()), 256, 0, ctx->stream>>>(p);
     CK(cudaGetLastError());
@@ -662,6 +662,8 @@ struct BatchWave {
     size_t first, count;          // instances
     size_t task_offset, n_tasks;  // tasks
 };
+
+constexpr size_t BATCH_SCRATCH_BYTES = (size_t)16 << 30;  // of a batch's waves, unless the caller says
 
 struct BatchPlan {
     std::vector<SgmInstance> descs;  // device path pointers filled in once the scratch is known
@@ -813,7 +815,7 @@ int run_batch(chiaro_depth_ctx *ctx, const chiaro_sgm_instance *in, size_t n, si
     } else {
         ctx->batch_key = 0;  // any other batch may move the scratch: the cached graph is void
         BatchPlan plan;
-        const size_t budget = scratch_bytes ? scratch_bytes : ((size_t)16 << 30);
+        const size_t budget = scratch_bytes ? scratch_bytes : BATCH_SCRATCH_BYTES;
         if (int st = plan_batch(in, n, budget / sizeof(float), plan)) return st;
         BatchDevice dev{};
         dev.scratch = dbuf<float>(ctx, "batch.paths", std::max<size_t>(plan.scratch_floats, 1));
@@ -1416,7 +1418,7 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     upload(ctx, g.labels, labels.data(), D);
     upload(ctx, g.spatial, sp.data(), sp.size());
     for (int t : g.targets) quad_plane(ctx, t, h_views[t]);
-    // the node tiles of a full-range cost volume; a banded search decides it for its fallback windows
+    // the node tiles of a full-range cost volume; a banded search decides on them for its fallback windows
     bool in_tiles = !spec && cost_in_tiles(ctx, h_views, reference, g.targets, o.near_depth, N, D);
     if (in_tiles) region_planes(ctx, h_views, reference, g.targets, o.near_depth);
     g.views = dbuf<DevView>(ctx, "coarse.views", n_views);
@@ -1445,11 +1447,12 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
     }
     launch_sample_planes(ctx, g.views, h_views, g.targets, true);
     g.h_views = h_views;
-    const auto tile_patches = [&] {
+    const auto tile_patches = [&](const int *nodes, size_t listed) {
         g.patches = dbuf<RefPatch>(ctx, "coarse_patches", N);
-        launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches}});
+        launch_patches(ctx, g.views, reference, {{g.columns, g.rows, g.step, radius, g.spatial, g.lattice, g.patches,
+                                                  nodes, (int)listed}});
     };
-    if (in_tiles) tile_patches();
+    if (in_tiles) tile_patches(nullptr, 0);
     CK(cudaEventRecord(ctx->events[1], s));
     uint8_t *tested = dbuf<uint8_t>(ctx, "coarse.tested", N);
     float *guidance = dbuf<float>(ctx, "coarse.guidance", N);
@@ -1565,17 +1568,30 @@ int run_coarse(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, int referenc
             float *wguid = dbuf<float>(ctx, "coarse.window_guidance", node_count);
             uint8_t *wtested = dbuf<uint8_t>(ctx, "coarse.window_tested", node_count);
             float *wagg = dbuf<float>(ctx, "coarse.window_aggregate", cost_floats);
-            in_tiles = cost_in_tiles(ctx, h_views, reference, g.targets, o.near_depth, N, D);
+            const bool whole = windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows;
+            // the paths of the SGM that follows: of the whole grid, or of the windows as one batch
+            // (run_batch), or if that goes in waves the band's, which are done with
+            CostScratch scratch{paths, 8 * pitch};
+            if (whole) {
+                scratch = sgm_path_planes(ctx, N * D);
+            } else {
+                size_t floats = 0;
+                for (const BandWindow &w : windows) floats += 8 * sgm_pitch((size_t)w.wc * w.wr * D);
+                if (floats <= BATCH_SCRATCH_BYTES / sizeof(float)) {
+                    ctx->batch_key = 0;  // as run_batch: a cached graph holds the old buffer
+                    scratch = {dbuf<float>(ctx, "batch.paths", floats), floats};
+                }
+            }
+            // by the windows' own size: a few windows of a large grid do not pay for the tiles' planes
+            in_tiles = scratch.floats >= (size_t)TILE_NODES * g.V * D &&
+                       cost_in_tiles(ctx, h_views, reference, g.targets, o.near_depth, node_count, D);
             if (in_tiles) {
                 region_planes(ctx, h_views, reference, g.targets, o.near_depth);
                 upload(ctx, g.views, h_views.data(), n_views);
                 launch_sample_planes(ctx, g.views, h_views, g.targets, false);
                 g.h_views = h_views;
-                tile_patches();
+                tile_patches(d_nodes, node_count);
             }
-            const bool whole = windows.size() == 1 && windows[0].wc == g.columns && windows[0].wr == g.rows;
-            // the band's paths are done with
-            const CostScratch scratch = whole ? sgm_path_planes(ctx, N * D) : CostScratch{paths, 8 * pitch};
             coarse_cost(ctx, g, reference, o, D, nullptr, nullptr, d_nodes, node_count, scratch, wscores, wcosts,
                         wguid, wtested);
             if (whole) {

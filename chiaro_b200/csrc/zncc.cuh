@@ -323,6 +323,8 @@ struct PatchGrid {
     const float *spatial;
     TapLattice lattice;  // of this grid, or planes == nullptr
     RefPatch *out;
+    const int *nodes;  // the nodes whose patches are wanted, `listed` of them, or nullptr: all
+    int listed;
 };
 struct PatchParams {
     const DevView *views;
@@ -332,8 +334,9 @@ struct PatchParams {
 
 __global__ void __launch_bounds__(256) patch_sums_kernel(PatchParams params) {
     const PatchGrid &p = params.grids[blockIdx.y];
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long)p.columns * p.rows) return;
+    long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (p.nodes ? (long)p.listed : (long)p.columns * p.rows)) return;
+    if (p.nodes) i = __ldg(p.nodes + i);
     const double cx = (double)((int)(i % p.columns) * p.step), cy = (double)((int)(i / p.columns) * p.step);
     const DevView &rv = params.views[params.reference];
     const TapLattice &lattice = p.lattice;
