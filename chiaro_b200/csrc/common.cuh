@@ -281,8 +281,9 @@ CH_HD bool grid_offset(double d, float g_lowest, float &e) {
     const int ex = ((int32_t)f2u(lowest) - 8) >> 23, eg = (int32_t)f2u(g_lowest) >> 23;  // negative: below 0
     const int k = ex - 25 < eg - 24 ? ex - 25 : eg - 24;                                 // w = 2^(k - 127)
     if (k < 107) return false;                                                           // w >= 2^-20
-    // r + f. d - 0.25 rounds only where |d| < 1/8, by at most 2^-55: far less than 2^-19 w, and
-    // where it lands on a multiple of w, s rounds to that multiple + 0.25 too (s >= 32)
+    // r + f. d - 0.25 rounds by at most 2^-53 |shift| < 2^-29 w (|q| < 2^24): far less than 2^-19 w.
+    // Where it so lands on a multiple of w, g + d lies within 2^-29 w of that multiple + 0.25; with
+    // w <= ulp32(s) / 4 = 2^27 ulp64(s) that is at most a quarter of s's own ulp, so s rounds to it too
     const double q = shift * u2d((uint64_t)(1023 + 127 - k) << 52);
     if (!(fabs(q) < 16777214.0)) return false;
 #ifdef __CUDA_ARCH__

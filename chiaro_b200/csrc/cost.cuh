@@ -13,17 +13,17 @@
 // stage (88% busy; about 11 passes a gather, the samples of a warp's labels lying in some 20
 // lines) and took 9.35 ms for 4160x3120, four targets, 129 labels. From the region a tap's four
 // shared loads take 7 to 8 passes (a warp's labels are 0.5 to 1.6 pixels apart, so some share a
-// bank) and the kernel is bound by instruction issue (68%) with the shared memory at 72%: 7.75 ms,
-// with the sample planes and patches 7.96. Two things decide that: the inner loops are not
+// bank) and the kernel is bound by instruction issue (68%) with the L1's data stage, which serves the
+// shared memory, at 77%: 7.75 ms, with the sample planes and patches 7.96. Two things decide that: the inner loops are not
 // unrolled (four-fold unrolled they missed the instruction cache, 9.58 ms), and the per-view
 // scores and the rare f64 displacements go to scratch in global memory, so that seven CTAs
 // stay resident (29 KB each).
 //
-// The same kernel scores a subset of the labels for the learned band: each node
-// scores `slots` labels, slot 0 being label 0 (the global warp) and the others
+// cost_volume_node_kernel, the form for small grids and planes, also scores a subset of the labels
+// for the learned band: each node scores `slots` labels, slot 0 being label 0 (the global warp) and the others
 // either one label list shared by every node (the band proposal's sampled labels)
-// or its tile's band [O, O + slots - 1); rows are then [N][slots]. A node list
-// restricts the CTAs to some nodes (the fallback windows), each writing the row
+// or its tile's band [O, O + slots - 1); rows are then [N][slots]. In either form
+// a node list restricts the CTAs to some nodes (the fallback windows), each writing the row
 // of its list position. A label's score and cost do not depend on which other
 // labels a node scores, so every subset holds the full volume's values bit for bit.
 #pragma once
@@ -58,7 +58,7 @@ struct CostParams {
     int places_per_block;
     float *scores, *costs, *guidance;
     uint8_t *tested;
-    // label subsets (slots == labels with no list and no bands: the full volume)
+    // label subsets (slots == labels with no list and no bands: the full volume; node tiles always)
     int slots;                  // labels scored per node; rows of the outputs
     const int *label_list;      // [slots]: slot -> label, or nullptr
     const int *band_first;      // [tiles_y][tiles_x]: slot s > 0 -> label band_first[tile] + s - 1, or nullptr
@@ -157,7 +157,6 @@ __device__ inline void aggregate_tile(const CostParams &p, const float *score, c
     for (int i = threadIdx.x; i < K * D; i += blockDim.x) {
         const int k = by_slots.quotient(i), slot = i - k * D, node = node_of[k];
         if (node < 0) continue;
-        const int label = cost_slot_label(p, node, slot);
         const float *views = score + k * V * D + slot;
         float agg = 0.0f;
         bool some;
@@ -174,7 +173,7 @@ __device__ inline void aggregate_tile(const CostParams &p, const float *score, c
         float cost;
         if (isfinite(total)) {
             tested[k] = 1;
-            float near_prior = label == 0 ? 0.0f : NEAR_DEPTH_PRIOR * (float)(label - 1) / (float)(p.labels - 2);
+            float near_prior = slot == 0 ? 0.0f : NEAR_DEPTH_PRIOR * (float)(slot - 1) / (float)(p.labels - 2);
             cost = clampf_r(1.0f - total, 0.0f, 2.0f) + near_prior;
         } else {
             cost = MISSING_COST;
@@ -334,10 +333,9 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
                     const int k = by_part.quotient(i), slot = first + i - k * slots, node = node_of[k];
                     item = k * D + slot;
                     if (node >= 0) {
-                        const int label = cost_slot_label(p, node, slot);
                         const ViewGeom &g = geom[k];
                         scored = g.gc_ok && g.taps_ok;
-                        if (scored && label > 0) scored = depth_delta(cam, g, p.label_depth[label], ddx, ddy);
+                        if (scored && slot > 0) scored = depth_delta(cam, g, p.label_depth[slot], ddx, ddy);
                         if (scored) {
                             TapRange r;
                             fast = taps_on_grid(box[k], ddx, ddy, tv.luma.width, tv.luma.height, offset, r);
@@ -405,9 +403,8 @@ __global__ void __launch_bounds__(T, 1024 / T) cost_volume_kernel(CostParams p, 
                     if (!fast && j - n_fast < p.places_per_block) {
                         at = places[j - n_fast];
                     } else {  // the region does not fit, or the scratch is full: the displacement again
-                        const int label = cost_slot_label(p, node_of[k], slot);
                         at = make_double2(0.0, 0.0);
-                        if (label > 0) depth_delta(cam, geom[k], p.label_depth[label], at.x, at.y);
+                        if (slot > 0) depth_delta(cam, geom[k], p.label_depth[slot], at.x, at.y);
                     }
                     const double2 place = make_double2(at.x * 0.5, at.y * 0.5);
                     if (fits && taps_inside(tap_range(box[k], place.x, place.y), tv.luma.width, tv.luma.height))

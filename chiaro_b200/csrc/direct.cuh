@@ -362,7 +362,7 @@ __device__ inline void warp_direct_scores(const DirectParams &p, const DirectSlo
 // node's items; the CTA then scores the pooled lists (every node's fast items,
 // then every node's exact items), so the lanes of all warps stay busy up to the
 // pool's last round instead of each node's; each warp then selects its node. It is bound by the
-// L1's data stage (82% of its cycles): with GRID items lie target by target, so that neighbouring
+// L1's data stage and instruction issue (each some 70% of its cycles): with GRID items lie target by target, so that neighbouring
 // lanes gather near one another (8.70 -> 8.51 ms at 4160x3120 with four targets). Without, on
 // planes small enough to lie in the L1, there is nothing to gain by that, and a target whose
 // patches cross an edge fills whole warps with the slower exact path: by candidate there (400x300,

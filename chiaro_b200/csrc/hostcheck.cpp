@@ -57,7 +57,8 @@ uint64_t chiaro_hc_exp_mismatches(uint32_t lo, uint32_t hi, double scale, uint32
 
 // grid_offset against the two-step f64 coordinate: random patches of positive half
 // positions and displacements (plain random ones, multiples of a power of two, and those
-// nudged by a few f64 ulps, where ties and their neighbours sit). Returns the mismatching
+// nudged by a few f64 ulps, where ties and their neighbours sit; and just inside a negative power of
+// two, where d - 0.25 itself rounds). Returns the mismatching
 // coordinates and counts the accepted patches.
 uint64_t chiaro_hc_grid_offset_mismatches(uint64_t patches, uint64_t seed, uint64_t *accepted) {
     uint64_t state = seed * 0x9E3779B97F4A7C15ull + 1, bad = 0;
@@ -72,8 +73,11 @@ uint64_t chiaro_hc_grid_offset_mismatches(uint64_t patches, uint64_t seed, uint6
     for (uint64_t i = 0; i < patches; ++i) {
         const double centre = std::exp2(unit() * 13.0);
         double d = (unit() * 2.0 - 1.0) * std::exp2(6.0 - unit() * (next() % 4 ? 4.0 : 60.0));
-        const int kind = (int)(next() % 4);
-        if (kind >= 2) {
+        const int kind = (int)(next() % 5);
+        if (kind == 4) {
+            d = -std::exp2((double)(next() % 9) - 2.0);
+            for (int k = 1 + (int)(next() % 15); k > 0; --k) d = std::nextafter(d, 0.0);
+        } else if (kind >= 2) {
             const double grid = std::exp2(-(double)(next() % 28));
             d = std::floor(d / grid) * grid;
             if (kind == 3)

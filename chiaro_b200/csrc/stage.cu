@@ -367,9 +367,8 @@ void set_smem_limits() {
 // 48 rows: 4160x3120, 129 labels took 9.96 / 9.97 / 9.24 / 9.71 ms at 32 / 40 / 48 / 56 rows
 // (fewer rows mean more parts, more rows fewer CTAs an SM). Tiles, cost volume of 2080x1560 with
 // 65 labels, two targets, at 1 / 2 / 4 / 8 nodes: 3.83 / 2.93 / 2.26 / 2.08 ms; 1567x1173 with 193
-// labels, three targets: 1.86 / 1.58 / 1.47 / 1.52 ms; 1040x780 with 17 labels, four targets: 0.64 /
-// 0.45 / 0.33 / 0.31 ms. Eight nodes pay for few labels, and a grid of few nodes takes smaller
-// tiles so that every SM has several (320x240, 25 labels: 0.127 ms at 2 nodes, 0.129 at 4 and 8).
+// labels, three targets: 1.86 / 1.58 / 1.47 / 1.52 ms. Eight nodes pay for few labels, and a grid of few
+// nodes takes smaller tiles so that every SM has several.
 constexpr int COST_REGION_ROWS = 48;
 
 void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_rows, int sm_count) {
@@ -395,15 +394,14 @@ void plan_cost_tiles(CostParams &p, const std::vector<DevView> &views, size_t n_
         p.passes[v] = 1;
         double dx, dy;
         if (!epipolar_extent(rv, tv, p.near_depth, dx, dy)) continue;
-        // the share of the segment that the scored labels cover, and the room for it beside the
-        // patch, the tile's nodes, the bilinear neighbour, alignment and the warp's own bending
-        const double share = p.band_first ? (double)p.slots / p.labels : 1.0;
+        // the room for the segment beside the patch, the tile's nodes, the bilinear neighbour,
+        // alignment and the warp's own bending
         const double fixed = 2 * p.radius + 8, step = p.step * 0.5;
         const double wide = (p.transposed[v] ? p.tile_h : p.tile_w) - 1, high = (p.transposed[v] ? p.tile_w : p.tile_h) - 1;
         const double room_wide = std::max(REGION_PITCH - 3 - fixed - wide * step, 8.0);
         const double room_high = std::max(p.region_rows - fixed - high * step, 8.0);
         // 64 samples are the reach of a hypothesis (depth.rs:1611-1613)
-        const double longest = std::max(dx, dy) * share;
+        const double longest = std::max(dx, dy);
         const double parts_wide = std::min(longest, 64.0) > room_wide ? longest / room_wide : 1.0;
         const double slope = std::min(dx, dy) / std::max(std::max(dx, dy), 1e-9);
         const double parts_high = std::min(longest, 64.0) * slope > room_high ? longest * slope / room_high : 1.0;
