@@ -61,6 +61,7 @@ struct chiaro_depth_ctx {
     std::string stage_key;     // key of the last device-buffer call
     uint64_t stage_key_epoch = 0;
     cudaGraphExec_t stage_exec = nullptr;
+    int stage_exec_launches = 0;  // that it holds
     int stage_graph_state = 0;  // last call: 0 launched, 1 captured, 2 replayed
     float timings[7] = {};
     int launches = 0;  // this library's kernel launches in the last stage call
@@ -1858,6 +1859,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         if (same && ctx->stage_exec) {
             CK(cudaGraphLaunch(ctx->stage_exec, s));
             ctx->stage_graph_state = 2;
+            ctx->launches = ctx->stage_exec_launches;
             rewritten = targets;
             if (V == 0) rewritten.clear();
             CK(cudaMemcpyAsync(&h_results, d_results, sizeof(Results), cudaMemcpyDeviceToHost, s));
@@ -2210,6 +2212,7 @@ void run_stage(chiaro_depth_ctx *ctx, std::vector<DevView> h_views, DevView *d_v
         }
         CK(cudaGraphLaunch(ctx->stage_exec, s));
         ctx->stage_graph_state = 1;
+        ctx->stage_exec_launches = ctx->launches;
     }
     if (ctx->stage_graph && !host && !debug) ctx->stage_key_epoch = ctx->alloc_epoch;
     if (host) {

@@ -85,8 +85,8 @@ def test_planes_beyond_the_f32_positions(ctx, width, sources):
     assert compare_with_the_oracle(ctx, scene, direct=True).any()
 
 
-@pytest.mark.parametrize("width,height,sources,planes", [(700, 520, 2, 96), (700, 520, 4, 96), (700, 520, 12, 96),
-                                                        (1000, 700, 9, 40)])
+@pytest.mark.parametrize("width,height,sources,planes", [(700, 520, 2, 96), (700, 520, 4, 96), (700, 520, 12, 30),
+                                                        (1000, 700, 9, 33)])
 def test_tiles_hold_no_scratch_of_their_own(width, height, sources, planes):
     """The same call with a lens that takes the tiles and with one that does not: the tiles add the
     nodes' reference patches (24 bytes each) and at most a copy of the targets' planes, and go in
@@ -95,12 +95,17 @@ def test_tiles_hold_no_scratch_of_their_own(width, height, sources, planes):
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from chiaro_b200.runtime import DepthContext
+    from oracle import oracle
     held = []
     for focal in (1200.0, 15000.0):
         scene = make_case(width, height, sources, planes, focal=focal)
         context = DepthContext(0)
         try:
-            assert compare_with_the_oracle(context, scene).any()
+            if not held:
+                assert compare_with_the_oracle(context, scene).any()
+            else:  # with the same debug outputs
+                (columns, rows, _), (cc, cr, _) = output_shape(width, height, scene.options)
+                run(context, scene, oracle.debug_buffers(sources + 1, cc * cr, planes + 1, columns * rows))
             held.append(context.memory_held())
         finally:
             context.close()
@@ -139,3 +144,17 @@ def test_a_limit_that_holds_the_other_form_is_enough(sources):
     for other in results[2:]:
         assert np.array_equal(other.depth.view(np.uint64), results[1].depth.view(np.uint64))
         assert np.array_equal(other.confidence.view(np.uint32), results[1].confidence.view(np.uint32))
+
+
+# 700x520: a CTA per target and a kernel that joins them
+@pytest.mark.parametrize("width,height,sources,planes", [(700, 520, 2, 96), (331, 250, 2, 24)])
+def test_a_replay_reports_the_launches_it_holds(ctx, width, height, sources, planes):
+    from chiaro_b200.depth import DeviceStage
+    scene = make_case(width, height, sources, planes)
+    stage = DeviceStage(scene.inputs(), 0, scene.alignments(), scene.options, context=ctx)
+    stage.graph = True
+    launches = []
+    for state in (0, 1, 2):  # launched, captured, replayed
+        assert stage() and stage.graph_state == state
+        launches.append(ctx.launches())
+    assert len(set(launches)) == 1
