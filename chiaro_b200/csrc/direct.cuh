@@ -462,8 +462,8 @@ __global__ void __launch_bounds__(256, 4) direct_depth_kernel(DirectParams p) {
 // left to the L1 cache. A copy of the taps (289 at the default radius, 8 bytes a target) is most
 // of a warp's shared memory, so on a large grid, where it leaves an SM fewer than
 // WIDE_LATTICE_WARPS, the taps are read from the tap lattice (LATTICE), as lines that neighbouring
-// nodes share, in as many warps as the registers allow (32 of 64 registers with GRID, 24 of 80
-// without). Each of its entries takes longer, so a grid below WIDE_LATTICE_NODES keeps the copy, nine
+// nodes share, in as many warps as the registers allow (24 of 80 registers; bounded to 64 they are 32
+// and spill: 1.85 against 1.77 ms, 4160x3120 with four targets). Each of its entries takes longer, so a grid below WIDE_LATTICE_NODES keeps the copy, nine
 // taps in flight a lane: its list is a round or two of warps, whose latency counts. Direct stage,
 // copy / lattice, in ms: 400x300 (7,676 fine nodes), three targets at radius 4, 0.22 / 0.24, four at
 // radius 8, 0.81 / 1.02; 1200x900 (67,951) with four at radius 4 0.91 / 0.95; 1600x1200 (120,701) with

@@ -258,7 +258,7 @@ int chiaro_refine_multiview_depth_device(chiaro_depth_ctx *ctx,
  * the reference; off by default). When enabled, a device-buffer call whose views
  * (pointers, sizes, flags, cameras), reference, options and output pointers equal the
  * previous call's is captured into a graph on its second occurrence and replayed from
- * the third on: the stage's ~35 launches become one, and a replay reads the current
+ * the third on: the stage's two dozen launches become one, and a replay reads the current
  * contents of the same buffers. Any other call, or any buffer the context reallocates
  * (another entry point on a larger size, for instance), voids the graph and the next
  * calls run, capture and replay afresh. Calls with debug arrays or host buffers never
