@@ -14,7 +14,7 @@
 // lines) and took 9.35 ms for 4160x3120, four targets, 129 labels. From the region a tap's four
 // shared loads take 7 to 8 passes (a warp's labels are 0.5 to 1.6 pixels apart, so some share a
 // bank) and the kernel is bound by instruction issue (68%) with the L1's data stage, which serves the
-// shared memory, at 77%: 7.75 ms, with the sample planes and patches 7.96. Two things decide that: the inner loops are not
+// shared memory, at 78%: 7.75 ms, with the sample planes and patches 7.96. Two things decide that: the inner loops are not
 // unrolled (four-fold unrolled they missed the instruction cache, 9.58 ms), and the per-view
 // scores and the rare f64 displacements go to scratch in global memory, so that seven CTAs
 // stay resident (29 KB each).
